@@ -404,6 +404,19 @@ int gr_host_matrix_check_gs_ring(const gr_host_matrix* h, int lower_only, gr_dty
   });
 }
 
+int gr_host_matrix_check_direct(const gr_host_matrix* h, int32_t sweep, int dilu, int32_t warps, int32_t* max_steps,
+                                int32_t* second, int32_t* in_place) {
+  return guarded([&] {
+    need(h, "matrix");
+    if (sweep < 0 || sweep > 2) gr::fail(GR_EINVAL, "sweep must be 0 (ILU), 1 (Gauss-Seidel) or 2 (Gauss-Seidel from zero)");
+    const gr::HostDirect D = gr::buildDirect(*h->m, static_cast<gr::RingKind>(sweep), dilu != 0, warps, h->m->valueType);
+    gr::checkDirect(*h->m, D);
+    if (max_steps) *max_steps = D.maxSteps - gr::kDirectHead - gr::kDirectAhead;
+    if (second) *second = D.second ? 1 : 0;
+    if (in_place) *in_place = D.gsInPlace ? 1 : 0;
+  });
+}
+
 int gr_host_matrix_set_spmv_layout(gr_host_matrix* h, int32_t layout) {
   return guarded([&] {
     need(h, "matrix");

@@ -40,8 +40,10 @@ struct SolverConfig {
   MultiColorMode solveMulticolor = MultiColorMode::Auto;
   MultiColorMode factorizeMulticolor = MultiColorMode::Auto;
   bool diagonalBased = false;
-  // Extension: substitution kernel, "auto" (the host-scheduled ring kernel
-  // when a tile fits shared memory, else the level-schedule kernel), "ring",
+  // Extension: substitution kernel, "auto" (the direct record kernel where
+  // directShape, solvers.cu, has it faster, else the host-scheduled ring kernel
+  // when a tile fits shared memory, else the level-schedule kernel; an option
+  // of the ring kernel selects that one), "ring",
   // "tma" (chunked byte ring with a producer warp), "warp" (warp per tile)
   // or "levels".
   int iluKernel = 0;  // 0 auto, 1 tma, 2 levels, 3 warp, 4 ring, 5 warp-per-tile ring
@@ -104,9 +106,10 @@ struct SolverConfig {
   // alpha, beta, omega and the convergence test in float, as the reference
   // computes them (float32 vectors only).
   bool reduceRef = false;
-  // Gauss-Seidel sweep kernel: 0 auto (the level ring with one warp per
-  // tile for float coefficients when a tile fits shared memory, a block per
-  // tile for double coefficients and in batches), 1
+  // Gauss-Seidel sweep kernel: 0 auto (the direct record kernel where
+  // directShape, solvers.cu, has it faster; else the level ring with one warp
+  // per tile for float coefficients when a tile fits shared memory, a block
+  // per tile for double coefficients and in batches), 1
   // the level ring with a block per tile, 2 level schedules in global
   // memory, 3 the level ring with one warp per tile.
   int gsKernel = 0;

@@ -336,6 +336,87 @@ struct LevelRing {
   DBuf haloStart, haloSrc;  // Gauss-Seidel rings
 };
 
+// Row records for the direct sweep kernels (kernels_direct.cu). A step is up
+// to 32 * warps rows of one level, thread q the q-th; rows of more than three
+// entries come first in their level (rows of a level are independent). The
+// records of a step form one block: per row {three values, two slots}, then
+// the rows' tails (third slot, row, diagonal), then, for the first `long`
+// rows of the step, the same of a second triple {three values, two slots} and
+// its third slot. Rows are padded to a multiple of kDirectAlign. A tile's
+// blocks follow one another in execution order (ILU: the forward sweep's,
+// then the backward sweep's), so a tile reads one contiguous stream, 16 to 24
+// bytes a row and sweep plus 20 for the long rows (an ILU(0) of a 7-point
+// grid: one in eight, because a tile numbers its separator rows last).
+//
+// Step word: rows (bits 0-7), the kDirect* flags, long rows (bits 10-17), the
+// block's size in 16-byte units (bits 18-31). A tile's table starts with {0,
+// forward steps, all steps, 0}; each sweep's steps are padded to a multiple
+// of kDirectUnroll by zero words, and the table ends in kDirectAhead zero
+// words.
+constexpr uint32_t kDirectEnd = 1u << 8;   // last step of its level: a barrier follows
+constexpr uint32_t kDirectDiag = 1u << 9;  // the rows have a diagonal (all but plain ILU's forward sweep)
+constexpr int kDirectLongShift = 10, kDirectUnitShift = 18;
+constexpr int kDirectHead = 4, kDirectUnroll = 4, kDirectAhead = 16;
+constexpr uint32_t kDirectAlign = 8;
+// Slots are stored as 4 x slot in 16 bits (the byte offset of a float).
+constexpr int kDirectMaxSlots = 16384;
+// Places within a block, in bytes, for values of V bytes: the triples (float:
+// one 16-byte word {v0, v1, v2, slots} a row; double: a plane of {v0, v1},
+// then one of {v2, slots, tail word}), the tails (float: {tail word, diagonal}
+// or the tail word; double: the diagonal), the second triples and their third
+// slots (float; in the tail word for double).
+template <int V>
+struct DirectBlock {
+  uint32_t plane, tail, second, plane2, third, bytes;
+  // diag: whether the step has kDirectDiag.
+  __host__ __device__ constexpr DirectBlock(uint32_t word, bool diag)
+      : plane(16u * padded(word & 0xFFu)),
+        tail((V == 4 ? 1u : 2u) * plane),
+        second(tail + plane / 16u * (V == 4 ? (diag ? 8u : 4u) : (diag ? 8u : 0u))),
+        plane2(16u * padded((word >> kDirectLongShift) & 0xFFu)),
+        third(second + (V == 4 ? 1u : 2u) * plane2),
+        bytes(third + (V == 4 ? plane2 / 4u : 0u)) {}
+  __host__ __device__ static constexpr uint32_t padded(uint32_t rows) {
+    return (rows + kDirectAlign - 1) & ~(kDirectAlign - 1);
+  }
+};
+struct HostDirect {
+  RingKind kind = RingKind::Ilu;
+  bool dilu = false, second = false, gsInPlace = false;  // second: some row has more than three entries
+  bool longForward = false;  // ILU: the forward sweep has such rows
+  i32 warps = 1, maxSteps = 0;
+  int valueBytes = 4;
+  i64 records = 0, units = 0, maxRows = 0, maxXSlots = 0;
+  // Per record (padding rows included): the CRS entries of the first
+  // triple's values (-1: padding) and its first two slots (4 c0 | 4 c1 <<
+  // 16); the third slot and the row (4 slot | 4 row << 16) in tail. second:
+  // the second triple's in src2 and its third slot in tail2.
+  std::vector<int4> src, src2;
+  std::vector<uint32_t> tail, tail2;
+  std::vector<uint32_t> steps;
+  std::vector<i32> stepStart;  // P + 1
+  // Per step word: the step's first record and the first 16-byte unit of its
+  // block.
+  std::vector<uint32_t> stepRecord, stepUnit;
+  std::vector<i32> haloStart, haloSrc;
+};
+// Whether the direct kernels can run a sweep of H (every row of the sweep
+// has at most 6 entries and a tile's slots fit 16 bits).
+bool directFits(const HostMatrix& H, RingKind kind);
+HostDirect buildDirect(const HostMatrix& H, RingKind kind, bool dilu, i32 warps, DType vt);
+// Replays the kernel's reads on the host: indices, block places, coverage,
+// entries and their order, and the dependency order between barriers.
+// Throws GR_EINVAL.
+void checkDirect(const HostMatrix& H, const HostDirect& D);
+struct DirectPlan {
+  RingKind kind = RingKind::Ilu;
+  bool dilu = false, second = false, gsInPlace = false;
+  bool longForward = false;  // ILU: the forward sweep has rows of more than three entries
+  i32 warps = 1, depth = 8, maxSteps = 0;  // depth: steps copied ahead
+  i64 records = 0, units = 0, maxRows = 0, maxXSlots = 0;
+  DBuf src, src2, tail, tail2, steps, stepStart, stepRecord, stepUnit, haloStart, haloSrc;
+};
+
 // Kinds of entries a schedule keeps per row.
 enum class SweepEntries {
   Lower,        // tile-local columns below the row, ascending (ILU forward)
@@ -400,6 +481,10 @@ struct DeviceMatrix {
       levelRings;  // [(dilu, ring bytes, group, compact allowed, kind, record levels)]
   LevelRing& levelRing(bool dilu, i64 ringBytes, i32 group, bool allowCompact = true,
                        RingKind kind = RingKind::Ilu, bool records = false);
+
+  std::map<std::tuple<int, bool, i32, i32>, std::unique_ptr<DirectPlan>> directPlans;  // [(kind, dilu, warps, depth)]
+  // nullptr when the direct kernels cannot run this sweep.
+  DirectPlan* directPlan(RingKind kind, bool dilu, i32 warps, i32 depth);
 
   // Device error word written by kernels whose bounded waits ran out
   // (GR_ETIMEOUT); 0 when clean.

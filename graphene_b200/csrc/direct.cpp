@@ -1,0 +1,358 @@
+// Host side of the direct sweep kernels (kernels_direct.cu): row records in
+// execution order and the step table of every tile. See HostDirect in
+// device.hpp for the layout.
+#include <algorithm>
+#include <atomic>
+
+#include "device.hpp"
+
+namespace gr {
+
+namespace {
+
+// Entries of tile-order row p (tile-local index il) in the order the sweep
+// subtracts them: lower ascending (ilu/Solver.cpp:391-403), upper descending
+// without halo (:424-436), or all in tile-local order
+// (gauss-seidel/Solver.cpp:76-79).
+template <class F>
+void eachEntry(const HostMatrix& H, RingKind kind, bool upper, i64 p, i64 il, i64 nRows, F&& f) {
+  const i64 b = H.rowPtr[p], e = H.rowPtr[p + 1];
+  if (kind == RingKind::GaussSeidel) {
+    for (i64 k = b; k < e; ++k) f(k);
+  } else if (upper) {
+    for (i64 k = e - 1; k >= b && H.colLocal[k] >= il; --k)
+      if (H.colLocal[k] < nRows) f(k);
+  } else {
+    for (i64 k = b; k < e && H.colLocal[k] <= il && H.colLocal[k] < nRows; ++k) f(k);
+  }
+}
+
+i64 blockBytes(int valueBytes, uint32_t word) {
+  const bool diag = (word & kDirectDiag) != 0;
+  return valueBytes == 4 ? DirectBlock<4>(word, diag).bytes : DirectBlock<8>(word, diag).bytes;
+}
+
+// Whether every in-tile entry above the diagonal lies in a later level than
+// its row, so that a sweep can overwrite the start values in place.
+bool sweepsInPlace(const HostMatrix& H) {
+  std::atomic<bool> ok{true};
+  parallelFor(H.P, [&](i64 T) {
+    const i64 base = H.tileStart[T], nRows = H.tileStart[T + 1] - base;
+    for (i64 r = 0; r < nRows && ok.load(std::memory_order_relaxed); ++r)
+      for (i64 k = H.rowPtr[base + r]; k < H.rowPtr[base + r + 1]; ++k) {
+        const i64 lc = H.colLocal[k];
+        if (lc > r && lc < nRows && H.lowerLevel[base + lc] <= H.lowerLevel[base + r]) {
+          ok = false;
+          break;
+        }
+      }
+  });
+  return ok;
+}
+
+i64 xSlotsOf(const HostMatrix& H, RingKind kind, bool inPlace, i64 T) {
+  const i64 nRows = H.tileStart[T + 1] - H.tileStart[T];
+  return kind == RingKind::GaussSeidel ? (inPlace ? 1 : 2) * nRows + H.tiles[T].nHalo + 1 : nRows + 1;
+}
+
+}  // namespace
+
+bool directFits(const HostMatrix& H, RingKind kind) {
+  for (i32 T = 0; T < H.P; ++T)
+    if (xSlotsOf(H, kind, false, T) > kDirectMaxSlots) return false;
+  std::atomic<bool> ok{true};
+  parallelChunks(H.P, [&](i64 t0, i64 t1) {
+    for (i64 T = t0; T < t1 && ok.load(std::memory_order_relaxed); ++T) {
+      const i64 base = H.tileStart[T], nRows = H.tileStart[T + 1] - base;
+      for (i64 r = 0; r < nRows; ++r) {
+        int c[2] = {0, 0};
+        for (int up = 0; up < (kind == RingKind::Ilu ? 2 : 1); ++up)
+          eachEntry(H, kind, up != 0, base + r, r, nRows, [&](i64) { ++c[up]; });
+        if (c[0] > 6 || c[1] > 6) ok = false;
+      }
+    }
+  }, 16);
+  return ok;
+}
+
+HostDirect buildDirect(const HostMatrix& H, RingKind kind, bool dilu, i32 warps, DType vt) {
+  const int threads = 32 * warps;
+  if (warps < 1 || warps == 3 || warps > 4) fail(GR_EINVAL, "direct sweeps run 1, 2 or 4 warps a tile");
+  if (!directFits(H, kind)) fail(GR_EUNSUPPORTED, "rows or tiles too large for the direct sweep");
+  const bool gs = kind != RingKind::Ilu;
+  HostDirect D;
+  D.kind = kind;
+  D.dilu = dilu;
+  D.warps = warps;
+  D.valueBytes = static_cast<int>(dtypeSize(vt));
+  D.gsInPlace = gs && (kind == RingKind::GaussSeidelLower || sweepsInPlace(H));
+  std::vector<std::vector<uint32_t>> tileSteps(H.P);
+  std::vector<std::vector<i32>> order(H.P);  // record -> tile-local row, -1: padding
+  std::vector<i64> nForward(H.P, 0);         // records of the forward sweep
+  std::atomic<bool> second{false}, longForward{false};
+  parallelFor(H.P, [&](i64 T) {
+    const i64 base = H.tileStart[T], nRows = H.tileStart[T + 1] - base;
+    std::vector<uint32_t>& st = tileSteps[T];
+    std::vector<i32>& ord = order[T];
+    st.assign(kDirectHead, 0u);
+    for (int sweep = 0; sweep < (gs ? 1 : 2); ++sweep) {
+      const bool upper = sweep == 1;
+      const std::vector<i32>& lev = upper ? H.upperLevel : H.lowerLevel;
+      const i32 nL = upper ? H.nUpperLevels[T] : H.nLowerLevels[T];
+      std::vector<i64> count(nL, 0), longs(nL, 0), next(nL, -1);
+      std::vector<char> isLong(nRows, 0);
+      for (i64 r = 0; r < nRows; ++r) {
+        const i32 l = lev[base + r];
+        ++count[l];
+        int c = 0;
+        eachEntry(H, kind, upper, base + r, r, nRows, [&](i64) { ++c; });
+        if (c > 3) {
+          second = true;
+          if (!upper) longForward = true;
+          isLong[r] = 1;
+          ++longs[l];
+        }
+      }
+      // Forward rows without entries keep their right-hand side: level 0 is
+      // left out.
+      i64 size = static_cast<i64>(ord.size());
+      for (i32 l = !gs && !upper && !dilu ? 1 : 0; l < nL; ++l) {
+        next[l] = size;
+        size += (count[l] + kDirectAlign - 1) / kDirectAlign * kDirectAlign;
+        for (i64 s = 0; s < count[l]; s += threads) {
+          const i64 k = std::min<i64>(threads, count[l] - s);
+          st.push_back(static_cast<uint32_t>(k) | (s + k == count[l] ? kDirectEnd : 0u) |
+                       (gs || upper || dilu ? kDirectDiag : 0u) |
+                       static_cast<uint32_t>(std::clamp<i64>(longs[l] - s, 0, k)) << kDirectLongShift);
+        }
+      }
+      while ((st.size() - kDirectHead) % kDirectUnroll != 0) st.push_back(0u);
+      st[upper || gs ? 2 : 1] = static_cast<uint32_t>(st.size() - kDirectHead);
+      ord.resize(size, -1);
+      for (const char want : {char(1), char(0)})  // long rows first
+        for (i64 r = 0; r < nRows; ++r)
+          if (i64& q = next[lev[base + r]]; q >= 0 && isLong[r] == want) ord[q++] = static_cast<i32>(r);
+      if (!upper) nForward[T] = size;
+    }
+    st.resize(st.size() + kDirectAhead, 0u);
+  });
+  D.second = second;
+  D.longForward = longForward;
+  D.stepStart.assign(H.P + 1, 0);
+  std::vector<i64> recStart(H.P + 1, 0);
+  for (i32 T = 0; T < H.P; ++T) {
+    recStart[T + 1] = recStart[T] + static_cast<i64>(order[T].size());
+    D.stepStart[T + 1] = D.stepStart[T] + static_cast<i32>(tileSteps[T].size());
+    D.maxSteps = std::max<i32>(D.maxSteps, static_cast<i32>(tileSteps[T].size()));
+    D.maxRows = std::max<i64>(D.maxRows, H.tileStart[T + 1] - H.tileStart[T]);
+    D.maxXSlots = std::max(D.maxXSlots, xSlotsOf(H, kind, D.gsInPlace, T));
+  }
+  D.records = recStart[H.P];
+  D.steps.reserve(D.stepStart[H.P]);
+  D.stepRecord.reserve(D.stepStart[H.P]);
+  D.stepUnit.reserve(D.stepStart[H.P]);
+  i64 rec = 0;
+  for (const auto& st : tileSteps)
+    for (size_t i = 0; i < st.size(); ++i) {
+      const uint32_t w = st[i];
+      const bool step = i >= static_cast<size_t>(kDirectHead);
+      const i64 rows = step ? (static_cast<i64>(w & 0xFFu) + kDirectAlign - 1) / kDirectAlign * kDirectAlign : 0;
+      const i64 units = step ? blockBytes(D.valueBytes, w) / 16 : 0;
+      D.steps.push_back(step ? w | static_cast<uint32_t>(units) << kDirectUnitShift : w);
+      D.stepRecord.push_back(static_cast<uint32_t>(rec));
+      D.stepUnit.push_back(static_cast<uint32_t>(D.units));
+      rec += rows;
+      D.units += units;
+    }
+  if (D.records >= (i64(1) << 31) || D.units >= (i64(1) << 32))
+    fail(GR_EUNSUPPORTED, "direct sweep exceeds 2^31 records");
+  const int4 none = make_int4(-1, -1, -1, 0);
+  D.src.assign(D.records, none);
+  D.tail.assign(D.records, 0u);
+  if (D.second) {
+    D.src2.assign(D.records, none);
+    D.tail2.assign(D.records, 0u);
+  }
+  parallelFor(H.P, [&](i64 T) {
+    const i64 base = H.tileStart[T], nRows = H.tileStart[T + 1] - base;
+    const i64 start = gs && !D.gsInPlace ? nRows : 0;  // where sweep-start values live
+    const uint32_t zero = static_cast<uint32_t>(4 * (xSlotsOf(H, kind, D.gsInPlace, T) - 1));
+    for (i64 q = 0; q < static_cast<i64>(order[T].size()); ++q) {
+      const i64 r = order[T][q], rec = recStart[T] + q;
+      if (r < 0) continue;
+      i32 e[6] = {-1, -1, -1, -1, -1, -1};
+      uint32_t c[6] = {zero, zero, zero, zero, zero, zero};
+      int m = 0;
+      eachEntry(H, kind, q >= nForward[T], base + r, r, nRows, [&](i64 k) {
+        const i64 lc = H.colLocal[k];
+        e[m] = static_cast<i32>(k);
+        c[m++] = static_cast<uint32_t>(4 * (gs && lc >= r ? start + lc : lc));
+      });
+      D.src[rec] = make_int4(e[0], e[1], e[2], static_cast<int>(c[0] | c[1] << 16));
+      D.tail[rec] = c[2] | static_cast<uint32_t>(4 * r) << 16;
+      if (D.second) {
+        D.src2[rec] = make_int4(e[3], e[4], e[5], static_cast<int>(c[3] | c[4] << 16));
+        D.tail2[rec] = c[5];
+      }
+    }
+  });
+  if (gs) D.haloStart.assign(H.P + 1, 0);  // sweeps from x = 0 read no halo
+  if (kind == RingKind::GaussSeidel) {
+    for (i32 T = 0; T < H.P; ++T) D.haloStart[T + 1] = D.haloStart[T] + static_cast<i32>(H.tiles[T].nHalo);
+    D.haloSrc.assign(D.haloStart[H.P], -1);
+    parallelFor(H.P, [&](i64 T) {
+      const i64 base = H.tileStart[T], nRows = H.tileStart[T + 1] - base;
+      for (i64 k = H.rowPtr[base]; k < H.rowPtr[base + nRows]; ++k)
+        if (H.colLocal[k] >= nRows) D.haloSrc[D.haloStart[T] + H.colLocal[k] - nRows] = H.colPerm[k];
+    });
+    for (i32 v : D.haloSrc)
+      if (v < 0) fail(GR_EINVAL, "direct sweep: a halo cell no entry reads");
+  }
+  return D;
+}
+
+void checkDirect(const HostMatrix& H, const HostDirect& D) {
+  const bool gs = D.kind != RingKind::Ilu;
+  const i64 threads = 32 * D.warps;
+  auto bad = [](i64 T, const std::string& what) {
+    fail(GR_EINVAL, "direct sweep check: tile " + std::to_string(T) + ": " + what);
+  };
+  if (static_cast<i64>(D.src.size()) != D.records || static_cast<i64>(D.tail.size()) != D.records ||
+      static_cast<i32>(D.stepStart.size()) != H.P + 1 || static_cast<i64>(D.steps.size()) != D.stepStart[H.P] ||
+      D.stepRecord.size() != D.steps.size() || D.stepUnit.size() != D.steps.size() ||
+      (D.second && (static_cast<i64>(D.src2.size()) != D.records || static_cast<i64>(D.tail2.size()) != D.records)))
+    fail(GR_EINVAL, "direct sweep check: table sizes");
+  parallelFor(H.P, [&](i64 T) {
+    const i64 base = H.tileStart[T], nRows = H.tileStart[T + 1] - base;
+    const i64 nHalo = D.kind == RingKind::GaussSeidel ? H.tiles[T].nHalo : 0;
+    const i64 start = gs && !D.gsInPlace ? nRows : 0;
+    const i64 slots = start + nRows + nHalo + 1;
+    if (gs && D.haloStart[T + 1] - D.haloStart[T] != nHalo) bad(T, "halo cells");
+    if (slots > D.maxXSlots || slots > kDirectMaxSlots || nRows > D.maxRows) bad(T, "slots");
+    const uint32_t* head = D.steps.data() + D.stepStart[T];
+    const i64 nS = D.stepStart[T + 1] - D.stepStart[T] - kDirectHead - kDirectAhead;
+    if (nS < 0 || nS + kDirectHead + kDirectAhead > D.maxSteps || head[2] != static_cast<uint32_t>(nS) ||
+        head[1] > head[2] || head[1] % kDirectUnroll != 0 || head[2] % kDirectUnroll != 0 || (gs && head[1] != 0))
+      bad(T, "steps");
+    const uint32_t* steps = head + kDirectHead;
+    for (i64 s = nS; s < nS + kDirectAhead; ++s)
+      if (steps[s] != 0) bad(T, "steps after the last");
+    if (gs) {
+      for (i64 h = 0; h < nHalo; ++h) {
+        const i32 src = D.haloSrc[D.haloStart[T] + h];
+        if (src < 0 || src >= H.n || (src >= base && src < base + nRows)) bad(T, "halo source");
+      }
+    }
+    // The level phase (barrier count) in which a row of the sweep was
+    // written, -1 before.
+    std::vector<i64> wroteLo(nRows, -1), wroteUp(nRows, -1);
+    // The kernel takes a tile's first block and adds up the steps' sizes.
+    i64 unit = D.stepUnit[D.stepStart[T]];
+    i64 phase = 0;
+    bool ended = true;
+    for (i64 s = 0; s < nS; ++s) {
+      const uint32_t w = steps[s];
+      const i64 k = w & 0xFFu;
+      const bool upper = !gs && s >= head[1];
+      if (!gs && s == head[1] && !ended) bad(T, "sweep order");
+      const i64 rows = (k + kDirectAlign - 1) / kDirectAlign * kDirectAlign;
+      const i64 nLong = (w >> kDirectLongShift) & 0xFFu, units = blockBytes(D.valueBytes, w) / 16;
+      i64 rec = D.stepRecord[D.stepStart[T] + kDirectHead + s];
+      if (k > threads || rec + rows > D.records || nLong > k || (nLong > 0 && !D.second) || (!gs && !upper && nLong > 0 && !D.longForward) ||
+          (w >> kDirectUnitShift) != units || unit + units > D.units ||
+          unit != D.stepUnit[D.stepStart[T] + kDirectHead + s])
+        bad(T, "step range");
+      unit += units;
+      if (k == 0 ? (!ended || w != 0) : ((w & kDirectDiag) != 0) != (gs || upper || D.dilu)) bad(T, "step flags");
+      if (k > 0) ended = false;
+      std::vector<i64>& wrote = upper ? wroteUp : wroteLo;
+      for (i64 q = 0; q < k; ++q, ++rec) {
+        const uint32_t tail = D.tail[rec];
+        const i64 r = (tail >> 16) / 4;
+        if (r >= nRows || wrote[r] >= 0 || (tail >> 16) % 4 != 0) bad(T, "row");
+        std::vector<i64> want, wantC;
+        eachEntry(H, D.kind, upper, base + r, r, nRows, [&](i64 e) {
+          want.push_back(e);
+          const i64 lc = H.colLocal[e];
+          wantC.push_back(4 * (gs && lc >= r ? start + lc : lc));
+        });
+        const int4 a = D.src[rec], b = D.second ? D.src2[rec] : make_int4(-1, -1, -1, 0);
+        const i64 e[6] = {a.x, a.y, a.z, b.x, b.y, b.z};
+        const uint32_t ca = static_cast<uint32_t>(a.w), cb = static_cast<uint32_t>(b.w);
+        const i64 c[6] = {ca & 0xFFFFu, ca >> 16, tail & 0xFFFFu, cb & 0xFFFFu, cb >> 16,
+                          D.second ? D.tail2[rec] : 0};
+        const size_t read = q < nLong ? 6 : 3;
+        if (want.size() > read) bad(T, "entries");
+        for (size_t j = 0; j < read; ++j) {
+          if (j >= want.size()) {
+            if (e[j] != -1 || c[j] != 4 * (slots - 1)) bad(T, "padding");
+            continue;
+          }
+          if (e[j] != want[j] || c[j] != wantC[j] || c[j] < 0 || c[j] >= 4 * (slots - 1)) bad(T, "entry");
+          const i64 lc = H.colLocal[want[j]];
+          if (lc >= nRows) continue;  // halo
+          if (gs && lc > r) {
+            if (D.gsInPlace && wroteLo[lc] >= 0) bad(T, "start value overwritten");
+            if (D.gsInPlace && H.lowerLevel[base + lc] <= H.lowerLevel[base + r]) bad(T, "start value in its level");
+          } else {
+            const i64 when = (upper ? wroteUp : wroteLo)[lc];
+            const bool leftOut = !upper && !gs && !D.dilu && H.lowerLevel[base + lc] == 0;
+            if (when >= phase || (when < 0 && !leftOut)) bad(T, "dependency order");
+          }
+        }
+        wrote[r] = phase;
+      }
+      if (w & kDirectEnd) {
+        ended = true;
+        ++phase;
+      }
+    }
+    if (!ended) bad(T, "after the last step");
+    for (i64 r = 0; r < nRows; ++r) {
+      if (wroteLo[r] < 0 && (gs || D.dilu || H.lowerLevel[base + r] != 0)) bad(T, "row not covered");
+      if (!gs && wroteUp[r] < 0) bad(T, "row not covered");
+    }
+  });
+}
+
+DirectPlan* DeviceMatrix::directPlan(RingKind kind, bool dilu, i32 warps, i32 depth) {
+  auto key = std::make_tuple(static_cast<int>(kind), dilu, warps, depth);
+  auto it = directPlans.find(key);
+  if (it != directPlans.end()) return it->second.get();
+  std::unique_ptr<DirectPlan> R;
+  if (directFits(*host, kind)) {
+    const HostDirect D = buildDirect(*host, kind, dilu, warps, vt);
+    R = std::make_unique<DirectPlan>();
+    R->kind = kind;
+    R->dilu = dilu;
+    R->second = D.second;
+    R->longForward = D.longForward;
+    R->gsInPlace = D.gsInPlace;
+    R->warps = warps;
+    R->depth = depth;
+    R->maxSteps = D.maxSteps;
+    R->records = D.records;
+    R->units = D.units;
+    R->maxRows = D.maxRows;
+    R->maxXSlots = D.maxXSlots;
+    R->src.upload(D.src);
+    R->tail.upload(D.tail);
+    if (D.second) {
+      R->src2.upload(D.src2);
+      R->tail2.upload(D.tail2);
+    }
+    R->steps.upload(D.steps);
+    R->stepStart.upload(D.stepStart);
+    R->stepRecord.upload(D.stepRecord);
+    R->stepUnit.upload(D.stepUnit);
+    if (kind != RingKind::Ilu) {
+      R->haloStart.upload(D.haloStart);
+      if (!D.haloSrc.empty()) R->haloSrc.upload(D.haloSrc);
+    }
+  }
+  DirectPlan* out = R.get();
+  directPlans[key] = std::move(R);
+  return out;
+}
+
+}  // namespace gr

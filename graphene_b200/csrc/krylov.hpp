@@ -102,6 +102,20 @@ void launchIluWarpRing(DeviceMatrix& A, const LevelRing& R, const void* stream, 
 void launchIluRing(DeviceMatrix& A, const LevelRing& R, const void* stream, bool dilu, const PrologueArgs& pro,
                    void* y, DType W, int l2Ahead, bool unroll, cudaStream_t s, bool pairRows = false, int computeWarps = 0,
                    bool waiter = true, bool producer = true);
+// Direct sweeps (kernels_direct.cu): shared memory of a block for vectors of
+// type W, the bytes of a solver's blocks (with what the kernels prefetch
+// beyond the last), their packing, and the
+// launches (launchGsDirect: the arguments of launchGsRing below).
+size_t iluDirectSmem(const DirectPlan& P, DType vt, DType W);
+size_t gsDirectSmem(const DirectPlan& P, DType vt, DType W);
+size_t directBytes(const DirectPlan& P);
+void launchDirectPack(DeviceMatrix& A, const DirectPlan& P, DBuf& data, const void* F, const void* inv,
+                      cudaStream_t s);
+void launchIluDirect(DeviceMatrix& A, const DirectPlan& P, const DBuf& data, bool dilu, const PrologueArgs& pro,
+                     void* y, DType W, cudaStream_t s);
+void launchGsDirect(DeviceMatrix& A, const DirectPlan& P, const DBuf& data, const PrologueArgs& pro, bool seedB,
+                    const void* xin, bool xinZero, void* xout, DType X, DType W, cudaStream_t s,
+                    bool dropHalo = false);
 // One Gauss-Seidel sweep through a Gauss-Seidel level ring (kernels_ring.cu):
 // xout from xin (xinZero: xin is all zeros and is not read; the ring may
 // then be a lower-only one). The right-hand side is the prologue's vector

@@ -24,9 +24,12 @@ i64 estimateFootprint(const HostMatrix& H, const std::string& json, DType t) {
   const i64 rows = n * (vs + 8) + 4 * (H.P + 1);                 // diagonal, tile starts, permutation
   const i64 localCrs = 4 * (n + 1) + m * (4 + vs);
   const i64 stream = 2 * (m * (4 + vs) + n * (8 + 2 * vs) + 64 * (i64(H.P) + 1));  // template + packed copy
+  // The direct sweeps' sources and packed records: at most 3 x 64 bytes a row
+  // and sweep, padding included.
+  const i64 direct = 2 * 192 * n;
   const i64 factors = m * vs + n * vs;
   const i64 vectors = 16 * n * std::max<i64>(8, static_cast<i64>(dtypeSize(t)));     // Krylov, MPIR, staging
-  return sell + rows + localCrs + stream + factors + vectors + (i64(4) << 20);
+  return sell + rows + localCrs + std::max(stream, direct) + factors + vectors + (i64(4) << 20);
 }
 
 struct Server::Entry {

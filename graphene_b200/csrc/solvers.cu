@@ -65,6 +65,59 @@ void printStats(const SolverConfig& c, const DeviceMatrix& A, const gr_stats& st
                st.iterations, st.converged ? "true" : "false", st.singular ? "true" : "false");
 }
 
+// Warps a tile and steps copied ahead of the direct sweep kernels
+// (kernels_direct.cu) for matrix A; {0, 0}: the level rings are the better
+// choice. What counts is how many tiles share an SM (t) and how many rows a
+// level has; results do not depend on the shape.
+//
+// ILU, float (us on B200, level ring -> direct; seven-point grids): with t <=
+// 1 a wide level needs the warps (64^3 / 64 tiles, 93 rows a level: 37.0 ->
+// 18.5 with four, 19.8 with two), a narrow one two (32^3 / 64 tiles, 23 rows:
+// 16.5 -> 8.2); between, two warps when a level fills them (128^3 / 512 tiles,
+// 93 rows: 45.5 -> 39.1), else one (96^3 / 432 tiles, 57 rows: 37.0 -> 20.6;
+// 64^3 / 512, 23 rows: 18.5 -> 10.3); with t > 4 one warp, copying 8 steps
+// ahead where all tiles then fit the SMs at once (128^3 / 1024: 41.1 -> 34.9),
+// 4 where only then they do (160^3 / 1370: 90.8 -> 80.5, with 8 104.6).
+// Double: the same with the two-warp line at 40 rows (128^3 / 1024: 66.9 ->
+// 53.3; 96^3 / 432: 37.0 -> 32.8).
+// When the tiles need clearly more than one wave, float tiles break even
+// (192^3 / 2368: 104.3 -> 103.0; MPIR there 139.3 -> 134.7 ms) and double ones
+// stay on the level ring (172.1 us against 188.4 at best).
+// Gauss-Seidel (two sweeps; a row costs a division and up to six entries, so
+// two warps from 45 rows a level on): float 128^3 / 1024 tiles 77.9 -> 66.5,
+// 160^3 / 1370 262.5 -> 156.6, 100^3 mesh / 1024 (36 rows) 49.2 -> 36.9, / 256
+// 82.0 -> 40.4; double mesh 86.0 -> 60.2 and 99.2 -> 63.2, but 128^3 / 1024
+// (1.7 waves) 155.6 -> 190.4.
+std::pair<i32, i32> directShape(const DeviceMatrix& A, RingKind kind) {
+  const HostMatrix& H = *A.host;
+  const bool gs = kind != RingKind::Ilu, f32 = A.vt == DType::F32;
+  i64 levels = 1, halo = 0;
+  for (i32 T = 0; T < H.P; ++T) {
+    levels += H.nLowerLevels[T];
+    halo = std::max(halo, H.tiles[T].nHalo);
+  }
+  const double t = static_cast<double>(H.P) / A.numSMs, rows = static_cast<double>(H.n) / static_cast<double>(levels);
+  i32 warps = 1, depth = gs ? 4 : 8;
+  if (gs) warps = t <= 2 ? 4 : rows > 45 ? 2 : 1;
+  else if (t <= 1) warps = rows > 40 ? 4 : 2;
+  else if (t <= 2) warps = 2;
+  else if (t <= 4) warps = rows > (f32 ? 72 : 40) ? 2 : 1;
+  // Whether all tiles are resident at once: the x slots (and the right-hand
+  // side), places for records with second triples, and about 2 KB of step
+  // table and reserve a block.
+  const i64 vs = f32 ? 4 : 8, rec = f32 ? 44 : 72;
+  const i64 fixed = vs * (gs ? 2 * H.maxTileRows + halo : H.maxTileRows) + 2048;
+  int perSM = 233472;
+  GR_CUDA(cudaDeviceGetAttribute(&perSM, cudaDevAttrMaxSharedMemoryPerMultiprocessor, A.device));
+  auto waves = [&](i32 d) {
+    const i64 slots = perSM / (fixed + rec * d * 32 * warps) * A.numSMs;
+    return slots > 0 ? static_cast<double>(H.P) / static_cast<double>(slots) : 1e9;
+  };
+  if (depth == 8 && waves(8) > 1 && waves(4) <= 1) depth = 4;
+  if (!f32 && waves(depth) > 1.25) return {0, 0};
+  return {warps, depth};
+}
+
 // ---------------------------------------------------------------------------
 class IluNode : public Node {
  public:
@@ -86,7 +139,15 @@ class IluNode : public Node {
         fail(GR_EUNSUPPORTED, "the warp ring ILU kernel does not fit this matrix's tiles in shared memory");
       kernel_ = 5;
     }
-    if (c.iluKernel == 0 || c.iluKernel == 4) {
+    if (c.iluKernel == 0 && !ringOptions(c)) {
+      const auto [warps, depth] = directShape(A, RingKind::Ilu);
+      DirectPlan* P = warps > 0 ? A.directPlan(RingKind::Ilu, dilu_, warps, depth) : nullptr;
+      if (P && iluDirectSmem(*P, A.vt, DType::F64) <= smemMax) {
+        kernel_ = 6;
+        direct_ = P;
+      }
+    }
+    if (kernel_ == 2 && (c.iluKernel == 0 || c.iluKernel == 4)) {
       LevelRing* R = nullptr;
       try {
         R = &A.levelRing(dilu_, c.ringBytes, c.tilesPerBlock > 0 ? c.tilesPerBlock : 1, c.compactRing,
@@ -113,7 +174,9 @@ class IluNode : public Node {
       else fail(GR_EUNSUPPORTED, "the requested ILU kernel does not fit this matrix's tiles in shared memory");
     }
     inv_.alloc(A.n * vs);
-    if (kernel_ == 4 || kernel_ == 5) {
+    if (kernel_ == 6) {
+      stream_.alloc(directBytes(*direct_));
+    } else if (kernel_ == 4 || kernel_ == 5) {
       stream_.alloc(std::max<i64>(16, ring_->bytes));
     } else if (kernel_ != 2) {
       SweepStream& S = A.iluSweepStream(dilu_);
@@ -143,7 +206,9 @@ class IluNode : public Node {
     launchIluFactor(A, dilu_ ? nullptr : F.get(), D.get(), A.offDiag.get(), dilu_, s());
     launchInvert(A, D.get(), inv_.get(), s());
     const void* vals = dilu_ ? A.offDiag.get() : F.get();
-    if (kernel_ == 4 || kernel_ == 5) {
+    if (kernel_ == 6) {
+      launchDirectPack(A, *direct_, stream_, vals, inv_.get(), s());
+    } else if (kernel_ == 4 || kernel_ == 5) {
       launchRingPack(A, *ring_, stream_.get(), vals, inv_.get(), s());
     } else if (kernel_ != 2) {
       launchStreamPack(A, *sweep_, stream_.get(), vals, inv_.get(), s());
@@ -154,7 +219,8 @@ class IluNode : public Node {
     GR_CUDA(cudaStreamSynchronize(s()));  // F and D are released on return
   }
   bool streamed() const { return sweep_ != nullptr; }
-  bool ringKernel() const { return kernel_ == 4; }
+  // Kernels that look up a block's system in a batch.
+  bool batchKernel() const { return kernel_ == 4 || kernel_ == 6; }
   gr_stats solve(void* x, const void* b, DType W, const KState* gate) override {
     PrologueArgs pro;
     pro.kind = Prologue::Plain;
@@ -166,7 +232,9 @@ class IluNode : public Node {
     return st;
   }
   void apply(const PrologueArgs& pro, void* y, DType W) {
-    if (kernel_ == 5)
+    if (kernel_ == 6)
+      launchIluDirect(A_, *direct_, stream_, dilu_, pro, y, W, s());
+    else if (kernel_ == 5)
       launchIluWarpRing(A_, *ring_, stream_.get(), dilu_, pro, y, W, cfg_.warpsPerBlock, cfg_.pairRows, s());
     else if (kernel_ == 4)
       launchIluRing(A_, *ring_, stream_.get(), dilu_, pro, y, W, cfg_.l2Ahead, cfg_.unrollRows != 0, s(),
@@ -220,7 +288,15 @@ class IluNode : public Node {
     autoWarps_ = 4;
   }
   int autoWarps_ = 0;  // compute warps chosen with automatic tile groups
-  int kernel_ = 2;  // 1 tma ring, 2 level schedule, 3 warp per tile, 4 host-scheduled ring, 5 its warp-per-tile form
+  // Whether the configuration sets an option of the ring kernel, which
+  // "auto" then runs.
+  static bool ringOptions(const SolverConfig& c) {
+    return c.ringBytes != 0 || c.l2Ahead != -1 || c.tilesPerBlock != 0 || !c.compactRing || !c.ringRecords ||
+           c.pairRows || c.computeWarps != 0 || !c.waitingWarp || !c.producerWarp || c.unrollRows != -1;
+  }
+  const DirectPlan* direct_ = nullptr;
+  // 1 tma ring, 2 level schedule, 3 warp per tile, 4 host-scheduled ring, 5 its warp-per-tile form, 6 direct records
+  int kernel_ = 2;
   int rowsPerLane_ = 2;
   DBuf inv_, Lval_, Uval_, stream_;
   const SweepStream* sweep_ = nullptr;
@@ -235,7 +311,17 @@ class GsNode : public Node {
     // The level-ring kernel when the tiles fit shared memory (for either
     // vector type): one ring with every entry, and one with the lower
     // entries only for sweeps that start from x = 0.
-    if (c.gsKernel != 2) {
+    if (c.gsKernel == 0 && c.ringRecords && c.warpsPerBlock == 1 && !c.gsPairRows) {
+      const auto [warps, depth] = directShape(A, RingKind::GaussSeidel);
+      DirectPlan* P = warps > 0 ? A.directPlan(RingKind::GaussSeidel, false, warps, depth) : nullptr;
+      DirectPlan* L = P ? A.directPlan(RingKind::GaussSeidelLower, false, warps, depth) : nullptr;
+      const size_t smemMax = static_cast<size_t>(maxDynamicSmem(A));
+      if (P && L && gsDirectSmem(*P, A.vt, DType::F64) <= smemMax && gsDirectSmem(*L, A.vt, DType::F64) <= smemMax) {
+        direct_ = P;
+        directLo_ = L;
+      }
+    }
+    if (c.gsKernel != 2 && !direct_) {
       try {
         ring_ = &A.levelRing(false, 0, 1, true, RingKind::GaussSeidel, c.ringRecords);
         ringLo_ = &A.levelRing(false, 0, 1, true, RingKind::GaussSeidelLower, c.ringRecords);
@@ -268,7 +354,10 @@ class GsNode : public Node {
         ring_ = ringLo_ = nullptr;
       }
     }
-    if (ring_) {
+    if (direct_) {
+      stream_.alloc(directBytes(*direct_));
+      streamLo_.alloc(directBytes(*directLo_));
+    } else if (ring_) {
       stream_.alloc(std::max<i64>(16, ring_->bytes));
       streamLo_.alloc(std::max<i64>(16, ringLo_->bytes));
     } else {
@@ -279,7 +368,10 @@ class GsNode : public Node {
   // Packs the matrix's current coefficients and diagonal into this
   // solver's level blocks.
   void refresh() override {
-    if (ring_) {
+    if (direct_) {
+      launchDirectPack(A_, *direct_, stream_, A_.offDiag.get(), A_.diag.get(), s());
+      launchDirectPack(A_, *directLo_, streamLo_, A_.offDiag.get(), A_.diag.get(), s());
+    } else if (ring_) {
       launchRingPack(A_, *ring_, stream_.get(), A_.offDiag.get(), A_.diag.get(), s());
       launchRingPack(A_, *ringLo_, streamLo_.get(), A_.offDiag.get(), A_.diag.get(), s());
     } else {
@@ -291,9 +383,9 @@ class GsNode : public Node {
   // Whether the first sweep can take PBiCGStab's p / s update as its
   // right-hand side (the level-ring kernel), and that application:
   // numFixedIterations sweeps from x = 0.
-  bool fusedPrologue() const { return ring_ != nullptr && cfg_.numFixedIterations > 0; }
-  // The block ring kernel (one block per tile, which batches need).
-  bool blockRing() const { return ring_ != nullptr && !warpRing_; }
+  bool fusedPrologue() const { return levelBlocks() && cfg_.numFixedIterations > 0; }
+  // A block per tile (which batches need).
+  bool blockPerTile() const { return direct_ != nullptr || (ring_ != nullptr && !warpRing_); }
   void applyFused(const PrologueArgs& pro, void* out, DType W) {
     ringSweeps(pro, out, W, cfg_.numFixedIterations, true);
   }
@@ -301,7 +393,7 @@ class GsNode : public Node {
   // Sweeps ping-pong between x and a scratch vector; the result ends in x.
   void sweeps(void* x, const void* b, DType W, int count, bool xZero, const KState* gate) {
     if (count <= 0) return;
-    if (ring_) {
+    if (levelBlocks()) {
       PrologueArgs pro;
       pro.kind = Prologue::Plain;
       pro.b = b;
@@ -391,7 +483,7 @@ class GsNode : public Node {
     if (Wc == W) return W;
     if (!(W == DType::F32 && Wc == DType::F64))
       fail(GR_EUNSUPPORTED, "GaussSeidel workingType must be the vectors' type or float64 over float32 vectors");
-    if (!ring_) fail(GR_EUNSUPPORTED, "a GaussSeidel workingType other than the vectors' needs the ring kernel");
+    if (!levelBlocks()) fail(GR_EUNSUPPORTED, "a GaussSeidel workingType other than the vectors' needs the ring kernel");
     return Wc;
   }
   // Level-ring sweeps: the first takes its right-hand side from `first`
@@ -409,13 +501,21 @@ class GsNode : public Node {
     void* other = tmp_.get();
     for (int k = 0; k < count; ++k) {
       const bool zero = xZero && k == 0;
-      launchGsRing(A_, zero ? *ringLo_ : *ring_, zero ? streamLo_.get() : stream_.get(), k == 0 ? first : plain,
+      if (direct_)
+        launchGsDirect(A_, zero ? *directLo_ : *direct_, zero ? streamLo_ : stream_, k == 0 ? first : plain,
+                       cfg_.gsSeedB, cur, zero, other, W, computeType(W), s(), cfg_.gsDropHalo);
+      else launchGsRing(A_, zero ? *ringLo_ : *ring_, zero ? streamLo_.get() : stream_.get(), k == 0 ? first : plain,
                    cfg_.gsSeedB, cur, zero, other, W, computeType(W), s(), warpRing_ ? cfg_.warpsPerBlock : 0,
                    cfg_.gsDropHalo, cfg_.gsPairRows);
       std::swap(cur, other);
     }
     if (cur != x) GR_CUDA(cudaMemcpyAsync(x, cur, A_.n * dtypeSize(W), cudaMemcpyDeviceToDevice, s()));
   }
+  // The kernels that read a solver's own packed rows (not the level
+  // schedules): the direct sweep and the level rings.
+  bool levelBlocks() const { return direct_ != nullptr || ring_ != nullptr; }
+  const DirectPlan* direct_ = nullptr;
+  const DirectPlan* directLo_ = nullptr;
   const LevelRing* ring_ = nullptr;
   const LevelRing* ringLo_ = nullptr;
   bool warpRing_ = false;  // one warp per tile (else one block per tile)
@@ -471,8 +571,8 @@ class PbicgstabNode : public Node {
       // A batch keeps one state per system; its preconditioner must look
       // up a block's system, which the block ring kernels (ILU substitution,
       // Gauss-Seidel sweeps) do.
-      const bool iluOk = ilu_ && ilu_->ringKernel();
-      const bool gsOk = gs_ && gs_->fusedPrologue() && gs_->blockRing();
+      const bool iluOk = ilu_ && ilu_->batchKernel();
+      const bool gsOk = gs_ && gs_->fusedPrologue() && gs_->blockPerTile();
       if (!iluOk && !gsOk)
         fail(GR_EUNSUPPORTED, "batched PBiCGStab needs the ILU preconditioner with the ring kernel, or Gauss-Seidel "
                               "with numFixedIterations > 0 on the block ring kernel");
@@ -613,7 +713,10 @@ class PbicgstabNode : public Node {
   DType graphType_ = DType::F32;
   int graphKernels_ = 0;
 
-  void* buf(int i) { return static_cast<char*>(vec_.get()) + static_cast<size_t>(i) * A_.n * dtypeSize(bufType_); }
+  // Vectors start at multiples of 64 elements, so that their 16-byte
+  // accesses are aligned whatever n is.
+  size_t stride() const { return (static_cast<size_t>(A_.n) + 63) / 64 * 64; }
+  void* buf(int i) { return static_cast<char*>(vec_.get()) + static_cast<size_t>(i) * stride() * dtypeSize(bufType_); }
   DBuf refTiles_;  // per-tile values of the reference-order reductions
   DBuf bw_;        // b in the working type (workingType float64 over float32 vectors)
   bool mixed_ = false, graphMixed_ = false;
@@ -626,7 +729,7 @@ class PbicgstabNode : public Node {
 
   void ensureBuffers(DType W) {
     if (haveBufs_ && bufType_ == W) return;
-    vec_.alloc(static_cast<size_t>(NBUF) * A_.n * dtypeSize(W));
+    vec_.alloc(static_cast<size_t>(NBUF) * stride() * dtypeSize(W));
     bufType_ = W;
     haveBufs_ = true;
     if (exec_) {

@@ -297,6 +297,18 @@ int gr_host_matrix_check_gs_ring(const gr_host_matrix* h, int lower_only, gr_dty
                                  int32_t allow_compact, int64_t* ring_bytes_used, int64_t* stream_bytes,
                                  int32_t* max_tile_levels, int32_t* in_place);
 
+/* The row records and step tables that the direct sweep kernels read (one
+ * block of `warps` (1, 2 or 4) warps per tile), built and replayed on the
+ * host: sweep 0 the ILU(0) / DILU forward and backward substitution, 1 a
+ * Gauss-Seidel sweep, 2 one from x = 0. Every row must be covered once, read
+ * its entries in order and only values that a barrier has published. Host
+ * only. Writes the most steps of a tile, whether any row has more than three
+ * entries, and whether the sweep runs in place. GR_EUNSUPPORTED for rows of
+ * more than six entries in a sweep or tiles of more than 16384 slots. No
+ * counterpart in the reference. */
+int gr_host_matrix_check_direct(const gr_host_matrix* h, int32_t sweep, int dilu, int32_t warps, int32_t* max_steps,
+                                int32_t* second, int32_t* in_place);
+
 /* DistributedTileLayout::loadVectorFromFile (DistributedTileLayout.cpp:185-206,
  * without halo): reads a MatrixMarket vector (a "vector" object, coordinate
  * or array, or the first column of a "matrix" object; unlisted entries are
