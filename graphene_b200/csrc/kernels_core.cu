@@ -412,7 +412,7 @@ void DeviceMatrix::makeBatch(const std::vector<i64>& rowBegin, const std::vector
     r1[s] = static_cast<i32>(rowBegin[s] + rowReal[s]);
     const i64 chunks = (rowReal[s] + 31) / 32;
     cBlocks[s] = static_cast<i32>(std::max<i64>(1, std::min<i64>((chunks + 7) / 8, sellGridCap())));
-    eBlocks[s] = static_cast<i32>(std::max<i64>(1, std::min<i64>(redBlocks, (rowReal[s] + 255) / 256)));
+    eBlocks[s] = static_cast<i32>(std::max<i64>(1, std::min<i64>(redBlocks, (rowReal[s] + 1023) / 1024)));
     cBlock0[s] = static_cast<i32>(cSys.size());
     eBlock0[s] = static_cast<i32>(eSys.size());
     for (int j = 0; j < cBlocks[s]; ++j) {
