@@ -399,6 +399,13 @@ struct HostDirect {
   // block.
   std::vector<uint32_t> stepRecord, stepUnit;
   std::vector<i32> haloStart, haloSrc;
+  // The factorisation in the forward sweep's order (ILU, when `factors`): per
+  // level {first record, rows | long rows << 16, first step word, first
+  // transpose}, tile T's levels from levelStart[T]; per forward record the
+  // CRS entries (column, row) of its entries (-1: none).
+  bool factors = false;
+  std::vector<i32> levelStart;
+  std::vector<int4> levels, transposed, transposed2;
 };
 // Whether the direct kernels can run a sweep of H (every row of the sweep
 // has at most 6 entries and a tile's slots fit 16 bits).
@@ -414,6 +421,8 @@ struct DirectPlan {
   bool longForward = false;  // ILU: the forward sweep has rows of more than three entries
   i32 warps = 1, depth = 8, maxSteps = 0;  // depth: steps copied ahead
   i64 records = 0, units = 0, maxRows = 0, maxXSlots = 0;
+  bool factors = false;
+  DBuf levelStart, levels, transposed, transposed2;
   DBuf src, src2, tail, tail2, steps, stepStart, stepRecord, stepUnit, haloStart, haloSrc;
 };
 

@@ -27,6 +27,33 @@ void eachEntry(const HostMatrix& H, RingKind kind, bool upper, i64 p, i64 il, i6
   }
 }
 
+// CRS entry (row p, tile-local column j), -1 when the pattern has none.
+i32 entryAt(const HostMatrix& H, i64 p, i64 j) {
+  for (i64 k = H.rowPtr[p]; k < H.rowPtr[p + 1]; ++k)
+    if (H.colLocal[k] == j) return static_cast<i32>(k);
+  return -1;
+}
+
+// Whether no tile has three rows that are pairwise coupled (a grid, a mesh of
+// hexahedra): ILU(0) then changes an entry only by its own division, and the
+// diagonal.
+bool triangleFree(const HostMatrix& H) {
+  std::atomic<bool> ok{true};
+  parallelFor(H.P, [&](i64 T) {
+    const i64 base = H.tileStart[T], nRows = H.tileStart[T + 1] - base;
+    for (i64 r = 0; r < nRows && ok.load(std::memory_order_relaxed); ++r) {
+      const i64 b = H.rowPtr[base + r], e = H.rowPtr[base + r + 1];
+      for (i64 k = b; k < e && H.colLocal[k] < r; ++k)
+        for (i64 j = k + 1; j < e && H.colLocal[j] < nRows; ++j)
+          if (entryAt(H, base + H.colLocal[k], H.colLocal[j]) >= 0) {
+            ok = false;
+            return;
+          }
+    }
+  });
+  return ok;
+}
+
 i64 blockBytes(int valueBytes, uint32_t word) {
   const bool diag = (word & kDirectDiag) != 0;
   return valueBytes == 4 ? DirectBlock<4>(word, diag).bytes : DirectBlock<8>(word, diag).bytes;
@@ -196,6 +223,44 @@ HostDirect buildDirect(const HostMatrix& H, RingKind kind, bool dilu, i32 warps,
       }
     }
   });
+  // The factorisation (DILU never changes an entry).
+  D.factors = !gs && (dilu || triangleFree(H));
+  if (D.factors) {
+    D.levelStart.assign(H.P + 1, 0);
+    std::vector<i64> forward(H.P + 1, 0);  // forward records before each tile
+    for (i32 T = 0; T < H.P; ++T) {
+      forward[T + 1] = forward[T] + nForward[T];
+      int4 level = make_int4(-1, 0, 0, 0);
+      for (uint32_t i = 0; i < D.steps[D.stepStart[T] + 1]; ++i) {
+        const i64 at = D.stepStart[T] + kDirectHead + i;
+        const uint32_t w = D.steps[at];
+        if ((w & 0xFFu) == 0) continue;
+        if (level.x < 0)
+          level = make_int4(static_cast<int>(D.stepRecord[at]), 0, static_cast<int>(at),
+                            static_cast<int>(forward[T] + D.stepRecord[at] - recStart[T]));
+        level.y += static_cast<int>((w & 0xFFu) | ((w >> kDirectLongShift) & 0xFFu) << 16);
+        if (w & kDirectEnd) {
+          D.levels.push_back(level);
+          level.x = -1;
+        }
+      }
+      D.levelStart[T + 1] = static_cast<i32>(D.levels.size());
+    }
+    D.transposed.assign(forward[H.P], none);
+    if (D.longForward) D.transposed2.assign(forward[H.P], none);
+    parallelFor(H.P, [&](i64 T) {
+      const i64 base = H.tileStart[T], nRows = H.tileStart[T + 1] - base;
+      for (i64 q = 0; q < nForward[T]; ++q) {
+        const i64 r = order[T][q];
+        if (r < 0) continue;
+        i32 t[6] = {-1, -1, -1, -1, -1, -1};
+        int m = 0;
+        eachEntry(H, kind, false, base + r, r, nRows, [&](i64 k) { t[m++] = entryAt(H, base + H.colLocal[k], r); });
+        D.transposed[forward[T] + q] = make_int4(t[0], t[1], t[2], 0);
+        if (D.longForward) D.transposed2[forward[T] + q] = make_int4(t[3], t[4], t[5], 0);
+      }
+    });
+  }
   if (gs) D.haloStart.assign(H.P + 1, 0);  // sweeps from x = 0 read no halo
   if (kind == RingKind::GaussSeidel) {
     for (i32 T = 0; T < H.P; ++T) D.haloStart[T + 1] = D.haloStart[T] + static_cast<i32>(H.tiles[T].nHalo);
@@ -308,6 +373,45 @@ void checkDirect(const HostMatrix& H, const HostDirect& D) {
       }
     }
     if (!ended) bad(T, "after the last step");
+    if (D.factors) {
+      // The levels cover the forward steps in order; an entry's transpose is
+      // the entry of its column's row, and no other entry of the two rows
+      // shares a column (not checked for DILU, which changes no entry).
+      i64 l = D.levelStart[T], at = D.stepStart[T] + kDirectHead;
+      const i64 stop = at + head[1];
+      for (; l < D.levelStart[T + 1]; ++l) {
+        const int4 v = D.levels[l];
+        if (at >= stop || v.z != at || v.x != static_cast<i64>(D.stepRecord[at])) bad(T, "level start");
+        i64 k = 0, nl = 0;
+        for (bool more = true; more; ++at) {
+          if (at >= stop || (k > 0 && k % threads != 0)) bad(T, "level steps");
+          if (static_cast<i64>(D.stepRecord[at]) != v.x + k) bad(T, "level records");
+          k += D.steps[at] & 0xFFu;
+          nl += (D.steps[at] >> kDirectLongShift) & 0xFFu;
+          more = (D.steps[at] & kDirectEnd) == 0;
+        }
+        if ((v.y & 0xFFFF) != k || (v.y >> 16) != nl) bad(T, "level rows");
+        for (i64 q = 0; q < k; ++q) {
+          const i64 r = (D.tail[v.x + q] >> 16) / 4;
+          const int4 a = D.transposed.at(v.w + q), b = D.longForward ? D.transposed2.at(v.w + q) : make_int4(-1, -1, -1, 0);
+          const i32 t[6] = {a.x, a.y, a.z, b.x, b.y, b.z};
+          int m = 0;
+          eachEntry(H, D.kind, false, base + r, r, nRows, [&](i64 e) {
+            const i64 c = H.colLocal[e];
+            const i64 p0 = H.rowPtr[base + c], p1 = H.rowPtr[base + c + 1];
+            if (t[m] < 0 ? entryAt(H, base + c, r) >= 0 : (t[m] < p0 || t[m] >= p1 || H.colLocal[t[m]] != r))
+              bad(T, "transpose");
+            for (i64 j = e + 1; !D.dilu && j < H.rowPtr[base + r + 1] && H.colLocal[j] < nRows; ++j)
+              if (entryAt(H, base + c, H.colLocal[j]) >= 0) bad(T, "fill-in");
+            ++m;
+          });
+          for (; m < 6; ++m)
+            if (t[m] != -1) bad(T, "transpose padding");
+        }
+      }
+      while (at < stop && D.steps[at] == 0) ++at;
+      if (at != stop) bad(T, "levels end");
+    }
     for (i64 r = 0; r < nRows; ++r) {
       if (wroteLo[r] < 0 && (gs || D.dilu || H.lowerLevel[base + r] != 0)) bad(T, "row not covered");
       if (!gs && wroteUp[r] < 0) bad(T, "row not covered");
@@ -340,6 +444,13 @@ DirectPlan* DeviceMatrix::directPlan(RingKind kind, bool dilu, i32 warps, i32 de
     if (D.second) {
       R->src2.upload(D.src2);
       R->tail2.upload(D.tail2);
+    }
+    R->factors = D.factors;
+    if (D.factors) {
+      R->levelStart.upload(D.levelStart);
+      R->levels.upload(D.levels);
+      R->transposed.upload(D.transposed);
+      if (D.longForward) R->transposed2.upload(D.transposed2);
     }
     R->steps.upload(D.steps);
     R->stepStart.upload(D.stepStart);

@@ -30,6 +30,7 @@ struct DirectView {
   const uint4* __restrict__ data;  // the steps' blocks
   int xSlots;   // slots of x in shared memory (a multiple of 4)
   int maxRows;  // rows of the largest tile
+  bool fetch;        // whether a block keeps its stream on its way to L2 ahead of its copies
   bool longForward;  // ILU: whether the forward sweep has rows of more than three entries
 };
 
@@ -323,6 +324,18 @@ __device__ __forceinline__ void levelBarrier() {
   else __syncthreads();
 }
 
+// 16-byte units of a tile's stream that its block keeps on their way to L2
+// beyond its copies. With the stream in DRAM the copies alone, DEPTH steps
+// ahead, leave too few bytes in flight: on B200, L2 flushed, 8 KB ahead ran
+// the 128^3 / 1024 ILU(0) in 41.3 us against 45.9 without (float64 63.6
+// against 68.3), 96^3 / 432 in 30.8 against 31.6, the 100^3 mesh's two sweeps
+// in 51.6 against 56.1; with it in L2 nothing changes (35.1 / 34.9 us; float64
+// 49.3 / 53.4). 4 and 16 KB ran within 3 us of it, a whole tile ahead slower.
+// Streams of less than 32 MB (kDirectFetchUnits) stay in L2 between a solve's
+// applications, and the 32^3 / 64 one takes 8.2 us without and up to 10 with
+// the prefetch, so they go without.
+constexpr uint32_t kDirectL2 = 512;
+
 // The copies, reads and barriers of a block's steps.
 template <class MV, class W, int NT, int WARPS, int DEPTH>
 struct DirectSteps {
@@ -331,6 +344,8 @@ struct DirectSteps {
   using S = DirectShape<MV, NT, THREADS, DEPTH>;
   using Rec = DirectRec<MV, NT>;
   const uint4* block;    // the next step's block to copy
+  const uint4* last;     // the end of the tile's blocks
+  uint32_t toFetch = 0;  // thread 0: units at its end that are not yet on their way to L2
   uint32_t steps;        // shared address of the next step's word
   uint32_t tid;
   uint32_t pa, pt, pc;   // shared addresses of the places of the current group of U steps
@@ -346,6 +361,12 @@ struct DirectSteps {
                                              tid, w);
     block += w >> kDirectUnitShift;
     copyCommit();
+  }
+  // Keeps kDirectL2 units beyond the next copy on their way to L2.
+  __device__ __forceinline__ void fetch() {
+    const uint32_t left = static_cast<uint32_t>(last - block), keep = left > kDirectL2 ? left - kDirectL2 : 0;
+    if (keep < toFetch) prefetchL2(last - toFetch, 16 * (toFetch - keep));
+    toFetch = keep;
   }
   template <int d>
   __device__ __forceinline__ void copyFirst(uint32_t w) {
@@ -366,6 +387,11 @@ struct DirectSteps {
     pt = s + S::tail + 8 * tid;
     pc = s + S::third + 4 * tid;
     block = V.data + __ldg(V.stepUnit + t0);
+    last = V.data + __ldg(V.stepUnit + V.stepStart[T + 1] - 1);
+    if (V.fetch && tid == 0) {
+      toFetch = static_cast<uint32_t>(last - block);
+      fetch();
+    }
     word = __ldg(table + kDirectHead);
     ahead = __ldg(table + kDirectHead + DEPTH);
     uint32_t w[DEPTH];
@@ -427,8 +453,9 @@ struct DirectSteps {
   // `count` steps, a multiple of U.
   template <bool LONG, bool DIAG2, bool LONG2, class F, class G>
   __device__ __forceinline__ void run(uint32_t count, unsigned char* x, F&& begin, G&& end) {
-    const uint32_t last = steps + 4 * count;
-    while (steps != last) {
+    const uint32_t stop = steps + 4 * count;
+    while (steps != stop) {
+      if (toFetch != 0) fetch();
       step<0, LONG, DIAG2, LONG2>(x, begin, end);
       step<1, LONG, DIAG2, LONG2>(x, begin, end);
       step<2, LONG, DIAG2, LONG2>(x, begin, end);
@@ -605,10 +632,184 @@ __global__ void __launch_bounds__(256) directPackKernel(const int* __restrict__ 
   }
 }
 
+// ILU(0) / DILU factorisation of every tile (ilu/Solver.cpp:167-218) for
+// patterns in which no entry (k, j) exists beside (i, k) and (i, j), written
+// straight into the solver's blocks. Row i then takes, for its lower entries
+// k in order, F_ik = A_ik / D_k and D_i -= F_ik F_ki; its other entries j only
+// lose F_ik times an absent entry's 0, which is 0 or, for an F_ik that is not
+// finite, NaN. The tile's D lies in shared memory, with each row's sum of
+// those zeros (z: +0, -0 or NaN). Rows run level by level in the forward
+// sweep's order, each thread a row; every gather is an index the host fixed.
+// It replaces a factorisation that searched global memory for each F_ki and
+// F_kj, a copy of the values, an inversion and a packing pass: on B200, 97 x
+// 96 x 95 rows in 432 tiles, 535 + 5 + 49 us for those kernels, 123 us for
+// this one (155 without the indices and values fetched ahead). What is left
+// is the chain of a level: up to three dependent divisions and a barrier.
+template <class MV, bool DILU>
+__global__ void __launch_bounds__(128) iluFactorDirectKernel(
+    const int* __restrict__ tileStart, const int* __restrict__ stepStart, const uint32_t* __restrict__ steps,
+    const uint32_t* __restrict__ stepRecord, const uint32_t* __restrict__ stepUnit, const int* __restrict__ levelStart,
+    const int4* __restrict__ levels, int stepShift, int maxRows, const int4* __restrict__ src,
+    const int4* __restrict__ src2, const uint32_t* __restrict__ tail, const uint32_t* __restrict__ tail2,
+    const int4* __restrict__ transposed, const int4* __restrict__ transposed2, const MV* __restrict__ A,
+    const MV* __restrict__ diag, uint4* __restrict__ data) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  MV* D = reinterpret_cast<MV*>(smem);
+  MV* z = D + maxRows;
+  const int T = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+  const int base = tileStart[T], nRows = tileStart[T + 1] - base;
+  for (int i = tid; i < nRows; i += 128) {
+    D[i] = diag[base + i];
+    z[i] = MV(0);
+  }
+  __syncthreads();
+  auto put = [&](char* out, uint32_t plane, const MV (&v)[3], int slots, uint32_t last) {
+    if constexpr (sizeof(MV) == 4) {
+      *reinterpret_cast<uint4*>(out) = make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]),
+                                                  static_cast<uint32_t>(slots));
+    } else {
+      *reinterpret_cast<uint4*>(out) =
+          make_uint4(__double2loint(v[0]), __double2hiint(v[0]), __double2loint(v[1]), __double2hiint(v[1]));
+      *reinterpret_cast<uint4*>(out + plane) =
+          make_uint4(__double2loint(v[2]), __double2hiint(v[2]), static_cast<uint32_t>(slots), last);
+    }
+  };
+  auto putTail = [&](char* tails, uint32_t q, uint32_t t, bool withDiag, MV inv) {
+    if constexpr (sizeof(MV) == 8) {
+      if (withDiag) reinterpret_cast<double*>(tails)[q] = inv;
+    } else {
+      if (withDiag) reinterpret_cast<uint2*>(tails)[q] = make_uint2(t, __float_as_uint(inv));
+      else reinterpret_cast<uint32_t*>(tails)[q] = t;
+    }
+  };
+  const int first = stepStart[T] + kDirectHead;
+  const int nForward = static_cast<int>(steps[first - kDirectHead + 1]);
+  const int4 none = make_int4(-1, -1, -1, 0);
+  // Row q of a level: its indices, the values they gather, and its
+  // elimination. Neither indices nor values depend on another row, so they
+  // are fetched two and one levels ahead; only D and z wait for the barrier.
+  struct Index {
+    int4 s, r, s2, r2;
+    uint32_t w, unit, t, t2;
+  };
+  struct Values {
+    MV v[6], u[6];
+  };
+  auto index = [&](const int4 lv, int q, Index& x) {
+    const bool on = q < (lv.y & 0xFFFF), two = q < (lv.y >> 16);
+    const int step = lv.z + (q >> stepShift);
+    x.w = on ? steps[step] : 0;
+    x.unit = on ? stepUnit[step] : 0;
+    x.t = on ? tail[lv.x + q] : 0;
+    x.s = on ? src[lv.x + q] : none;
+    x.r = on ? transposed[lv.w + q] : none;
+    x.s2 = two ? src2[lv.x + q] : none;
+    x.r2 = two ? transposed2[lv.w + q] : none;
+    x.t2 = two ? tail2[lv.x + q] : 0;
+  };
+  auto gather = [&](const Index& x, Values& g) {
+    const int e[6] = {x.s.x, x.s.y, x.s.z, x.s2.x, x.s2.y, x.s2.z}, et[6] = {x.r.x, x.r.y, x.r.z, x.r2.x, x.r2.y, x.r2.z};
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      g.v[k] = e[k] >= 0 ? A[e[k]] : MV(0);
+      g.u[k] = et[k] >= 0 ? A[et[k]] : MV(0);
+    }
+  };
+  auto eliminate = [&](const int4 lv, int q, const Index& x, Values& g) {
+    const int e[6] = {x.s.x, x.s.y, x.s.z, x.s2.x, x.s2.y, x.s2.z}, et[6] = {x.r.x, x.r.y, x.r.z, x.r2.x, x.r2.y, x.r2.z};
+    const uint32_t sw = static_cast<uint32_t>(x.s.w), sw2 = static_cast<uint32_t>(x.s2.w);
+    const uint32_t c[6] = {sw & 0xFFFFu, sw >> 16, x.t & 0xFFFFu, sw2 & 0xFFFFu, sw2 >> 16, x.t2};
+    MV d = D[x.t >> 18], zi = MV(0);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      if (e[k] < 0) continue;
+      const MV dk = D[c[k] >> 2];
+      if (DILU) {
+        d = sub(d, dvd(mul(g.v[k], g.u[k]), dk));
+      } else {
+        g.v[k] = dvd(g.v[k], dk);
+        const MV zk = mul(g.v[k], MV(0));
+#pragma unroll
+        for (int j = k + 1; j < 6; ++j)
+          if (e[j] >= 0) g.v[j] = sub(g.v[j], zk);
+        if (zi == zi && (zk != zk || signbit(zk))) zi = zk;
+        d = sub(d, mul(g.v[k], et[k] >= 0 ? sub(g.u[k], z[c[k] >> 2]) : MV(0)));
+      }
+    }
+    D[x.t >> 18] = d;
+    z[x.t >> 18] = zi;
+    const uint32_t at = static_cast<uint32_t>(q) & ((1u << stepShift) - 1);
+    const DirectBlock<sizeof(MV)> blk(x.w, DILU);
+    char* out = reinterpret_cast<char*>(data + x.unit);
+    const MV lo[3] = {g.v[0], g.v[1], g.v[2]}, hi[3] = {g.v[3], g.v[4], g.v[5]};
+    put(out + 16 * at, blk.plane, lo, x.s.w, x.t);
+    putTail(out + blk.tail, at, x.t, DILU, DILU ? dvd(MV(1), d) : d);
+    if (q < (lv.y >> 16)) {
+      put(out + blk.second + 16 * at, blk.plane2, hi, x.s2.w, x.t2);
+      if (sizeof(MV) == 4) reinterpret_cast<uint32_t*>(out + blk.third)[at] = x.t2;
+    }
+  };
+  const int l0 = levelStart[T], l1 = levelStart[T + 1];
+  auto level = [&](int l) { return l < l1 ? levels[l] : make_int4(0, 0, 0, 0); };
+  int4 lv = level(l0), lv1 = level(l0 + 1);
+  Index x, x1;
+  Values g;
+  index(lv, tid, x);
+  index(lv1, tid, x1);
+  gather(x, g);
+  for (int l = l0; l < l1; ++l) {
+    Values g1;
+    gather(x1, g1);
+    const int4 lv2 = level(l + 2);
+    if (tid < (lv.y & 0xFFFF)) eliminate(lv, tid, x, g);
+    x = x1;
+    index(lv2, tid, x1);
+    for (int q = tid + 128; q < (lv.y & 0xFFFF); q += 128) {  // wide levels
+      Index xq;
+      Values gq;
+      index(lv, q, xq);
+      gather(xq, gq);
+      eliminate(lv, q, xq, gq);
+    }
+    g = g1;
+    lv = lv1;
+    lv1 = lv2;
+    __syncthreads();
+  }
+  for (int i = tid; i < nRows; i += 128) D[i] = dvd(MV(1), D[i]);
+  __syncthreads();
+  // The backward records: a warp per step.
+  const int stop = stepStart[T + 1];
+#pragma unroll 2
+  for (int i = first + nForward + (tid >> 5); i < stop; i += 4) {
+    const uint32_t w = steps[i], rows = w & 0xFFu, longs = (w >> kDirectLongShift) & 0xFFu;
+    const DirectBlock<sizeof(MV)> blk(w, true);
+    char* out = reinterpret_cast<char*>(data + stepUnit[i]);
+    for (uint32_t q = lane; q < rows; q += 32) {
+      const size_t p = stepRecord[i] + q;
+      const uint32_t t = tail[p];
+      const MV zi = DILU ? MV(0) : z[t >> 18];
+      auto val = [&](int e) { return e < 0 ? MV(0) : DILU ? A[e] : sub(A[e], zi); };
+      const int4 s = src[p];
+      const MV lo[3] = {val(s.x), val(s.y), val(s.z)};
+      put(out + 16 * q, blk.plane, lo, s.w, t);
+      putTail(out + blk.tail, q, t, true, D[t >> 18]);
+      if (q < longs) {
+        const int4 s2 = src2[p];
+        const MV hi[3] = {val(s2.x), val(s2.y), val(s2.z)};
+        put(out + blk.second + 16 * q, blk.plane2, hi, s2.w, tail2[p]);
+        if (sizeof(MV) == 4) reinterpret_cast<uint32_t*>(out + blk.third)[q] = tail2[p];
+      }
+    }
+  }
+}
+
 }  // namespace dev
 
 // ---------------------------------------------------------------------------
 namespace {
+
+constexpr i64 kDirectFetchUnits = (i64(32) << 20) / 16;
 
 dev::DirectView directView(const DeviceMatrix& A, const DirectPlan& P, const DBuf& data) {
   return dev::DirectView{A.tileStart.as<int>(),
@@ -618,6 +819,7 @@ dev::DirectView directView(const DeviceMatrix& A, const DirectPlan& P, const DBu
                          data.as<uint4>(),
                          static_cast<int>((P.maxXSlots + 3) / 4 * 4),
                          static_cast<int>(P.maxRows),
+                         P.units >= kDirectFetchUnits,
                          P.longForward};
 }
 
@@ -654,6 +856,29 @@ void launchDirectPack(DeviceMatrix& A, const DirectPlan& P, DBuf& data, const vo
   if (A.vt == DType::F32) go(0.0f);
   else go(0.0);
   checkLaunch("direct_pack");
+}
+
+size_t directFactorSmem(const DirectPlan& P, DType vt) { return 2 * static_cast<size_t>(P.maxRows) * dtypeSize(vt); }
+
+void launchIluFactorDirect(DeviceMatrix& A, const DirectPlan& P, DBuf& data, bool dilu, cudaStream_t s) {
+  if (!P.factors || P.dilu != dilu) fail(GR_EINVAL, "the plan does not factorise this matrix");
+  const size_t smem = directFactorSmem(P, A.vt);
+  const int stepShift = P.warps == 1 ? 5 : P.warps == 2 ? 6 : 7;
+  auto go = [&](auto zero) {
+    using MV = decltype(zero);
+    auto kernel = dilu ? dev::iluFactorDirectKernel<MV, true> : dev::iluFactorDirectKernel<MV, false>;
+    ensureDynamicSmem(reinterpret_cast<const void*>(kernel), smem);
+    preferSharedCarveout(reinterpret_cast<const void*>(kernel));
+    kernel<<<A.P, 128, smem, s>>>(
+        A.tileStart.as<int>(), P.stepStart.as<int>(), P.steps.as<uint32_t>(), P.stepRecord.as<uint32_t>(),
+        P.stepUnit.as<uint32_t>(), P.levelStart.as<int>(), P.levels.as<int4>(), stepShift, static_cast<int>(P.maxRows),
+        P.src.as<int4>(), P.second ? P.src2.as<int4>() : nullptr, P.tail.as<uint32_t>(),
+        P.second ? P.tail2.as<uint32_t>() : nullptr, P.transposed.as<int4>(),
+        P.longForward ? P.transposed2.as<int4>() : nullptr, A.offDiag.as<MV>(), A.diag.as<MV>(), data.as<uint4>());
+  };
+  if (A.vt == DType::F32) go(0.0f);
+  else go(0.0);
+  checkLaunch("ilu_factor_direct");
 }
 
 namespace {

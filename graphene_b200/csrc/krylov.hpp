@@ -111,6 +111,10 @@ size_t gsDirectSmem(const DirectPlan& P, DType vt, DType W);
 size_t directBytes(const DirectPlan& P);
 void launchDirectPack(DeviceMatrix& A, const DirectPlan& P, DBuf& data, const void* F, const void* inv,
                       cudaStream_t s);
+// The factorisation of the matrix's values straight into the blocks (plans
+// with `factors`), and its shared memory.
+size_t directFactorSmem(const DirectPlan& P, DType vt);
+void launchIluFactorDirect(DeviceMatrix& A, const DirectPlan& P, DBuf& data, bool dilu, cudaStream_t s);
 void launchIluDirect(DeviceMatrix& A, const DirectPlan& P, const DBuf& data, bool dilu, const PrologueArgs& pro,
                      void* y, DType W, cudaStream_t s);
 void launchGsDirect(DeviceMatrix& A, const DirectPlan& P, const DBuf& data, const PrologueArgs& pro, bool seedB,

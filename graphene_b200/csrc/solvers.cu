@@ -74,17 +74,18 @@ void printStats(const SolverConfig& c, const DeviceMatrix& A, const gr_stats& st
 // 1 a wide level needs the warps (64^3 / 64 tiles, 93 rows a level: 37.0 ->
 // 18.5 with four, 19.8 with two), a narrow one two (32^3 / 64 tiles, 23 rows:
 // 16.5 -> 8.2); between, two warps when a level fills them (128^3 / 512 tiles,
-// 93 rows: 45.5 -> 39.1), else one (96^3 / 432 tiles, 57 rows: 37.0 -> 20.6;
-// 64^3 / 512, 23 rows: 18.5 -> 10.3); with t > 4 one warp, copying 8 steps
+// 93 rows: 45.5 -> 39.1; 96^3 / 432, 57 rows: 36.9 -> 22.6, with the records in
+// DRAM 44.2 -> 30.8, one warp 32.8), else one (64^3 / 512, 23 rows: 18.5 ->
+// 10.3); with t > 4 one warp, copying 8 steps
 // ahead where all tiles then fit the SMs at once (128^3 / 1024: 41.1 -> 34.9),
 // 4 where only then they do (160^3 / 1370: 90.8 -> 80.5, with 8 104.6).
-// Double: the same with the two-warp line at 40 rows (128^3 / 1024: 66.9 ->
-// 53.3; 96^3 / 432: 37.0 -> 32.8).
+// Double: 128^3 / 1024 66.9 -> 49.3, 96^3 / 432 37.0 -> 32.8.
 // When the tiles need clearly more than one wave, float tiles break even
 // (192^3 / 2368: 104.3 -> 103.0; MPIR there 139.3 -> 134.7 ms) and double ones
 // stay on the level ring (172.1 us against 188.4 at best).
 // Gauss-Seidel (two sweeps; a row costs a division and up to six entries, so
-// two warps from 45 rows a level on): float 128^3 / 1024 tiles 77.9 -> 66.5,
+// float tiles take two warps from 45 rows a level on; double tiles, of which
+// fewer fit an SM, one: the mesh with two 82.9): float 128^3 / 1024 tiles 77.9 -> 66.5,
 // 160^3 / 1370 262.5 -> 156.6, 100^3 mesh / 1024 (36 rows) 49.2 -> 36.9, / 256
 // 82.0 -> 40.4; double mesh 86.0 -> 60.2 and 99.2 -> 63.2, but 128^3 / 1024
 // (1.7 waves) 155.6 -> 190.4.
@@ -98,10 +99,10 @@ std::pair<i32, i32> directShape(const DeviceMatrix& A, RingKind kind) {
   }
   const double t = static_cast<double>(H.P) / A.numSMs, rows = static_cast<double>(H.n) / static_cast<double>(levels);
   i32 warps = 1, depth = gs ? 4 : 8;
-  if (gs) warps = t <= 2 ? 4 : rows > 45 ? 2 : 1;
+  if (gs) warps = t <= 2 ? 4 : f32 && rows > 45 ? 2 : 1;
   else if (t <= 1) warps = rows > 40 ? 4 : 2;
   else if (t <= 2) warps = 2;
-  else if (t <= 4) warps = rows > (f32 ? 72 : 40) ? 2 : 1;
+  else if (t <= 4) warps = rows > 40 ? 2 : 1;
   // Whether all tiles are resident at once: the x slots (and the right-hand
   // side), places for records with second triples, and about 2 KB of step
   // table and reserve a block.
@@ -173,7 +174,8 @@ class IluNode : public Node {
       else if (c.iluKernel == 1 && tmaFits) kernel_ = 1;
       else fail(GR_EUNSUPPORTED, "the requested ILU kernel does not fit this matrix's tiles in shared memory");
     }
-    inv_.alloc(A.n * vs);
+    fusedFactor_ = kernel_ == 6 && direct_->factors && directFactorSmem(*direct_, A.vt) <= smemMax;
+    if (!fusedFactor_) inv_.alloc(A.n * vs);
     if (kernel_ == 6) {
       stream_.alloc(directBytes(*direct_));
     } else if (kernel_ == 4 || kernel_ == 5) {
@@ -195,6 +197,11 @@ class IluNode : public Node {
   // level blocks (the buffers allocated at construction).
   void factorAndPack() {
     DeviceMatrix& A = A_;
+    if (fusedFactor_) {
+      launchIluFactorDirect(A, *direct_, stream_, dilu_, s());
+      GR_CUDA(cudaStreamSynchronize(s()));
+      return;
+    }
     const size_t vs = dtypeSize(A.vt);
     DBuf F, D;
     if (!dilu_) {
@@ -295,6 +302,7 @@ class IluNode : public Node {
            c.pairRows || c.computeWarps != 0 || !c.waitingWarp || !c.producerWarp || c.unrollRows != -1;
   }
   const DirectPlan* direct_ = nullptr;
+  bool fusedFactor_ = false;  // factorises straight into the direct sweep's blocks
   // 1 tma ring, 2 level schedule, 3 warp per tile, 4 host-scheduled ring, 5 its warp-per-tile form, 6 direct records
   int kernel_ = 2;
   int rowsPerLane_ = 2;

@@ -141,3 +141,37 @@ def test_direct_sweeps_equal_level_schedules(name, types):
             gb.Solver(A, {"type": "PBiCGStab", "maxIterations": 4, "preconditioner": {**pre, **kernel}}).solve(x, b[:n])
             xs.append(x)
         assert torch.equal(*xs), pre
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("dilu", [False, True])
+@pytest.mark.parametrize("first_rows", [False, True])
+def test_factorisation_of_zeros_and_infinities(dtype, dilu, first_rows):
+    """A zero diagonal, signed zeros and overflowing quotients go through the
+    factorisation as through the level-scheduled one: the same bits, NaN where
+    it has NaN."""
+    import torch
+    h = gb.generate3DPoissonMatrix(gb.parseType(dtype), 9, 8, 7, 6, gb.PART_RCB)
+    rp, col, off, dg = h.globalCrs()
+    rng = np.random.default_rng(5)
+    off = off * rng.uniform(0.5, 2.0, len(off))
+    off[rng.integers(0, len(off), 40)] = -0.0
+    off[rng.integers(0, len(off), 10)] = 1e38 if dtype == "float32" else 1e308
+    dg = dg.copy()
+    dg[rng.integers(0, len(dg), 4)] = 0.0
+    dg[rng.integers(0, len(dg), 4)] = 1e-38 if dtype == "float32" else 1e-308
+    if first_rows:  # rows that others divide by before anything is subtracted from them
+        lower = h.levels()[0]
+        natural = h.decomposeVector(np.arange(h.numRows, dtype=np.float64), gb.FLOAT64).astype(int)
+        dg[natural[lower == 0][:3]] = 0.0
+    A = h.copyToTile()
+    A.updateGlobalValues(off, dg)
+    b = torch.from_numpy(rng.uniform(-1, 1, h.numRows)).to(getattr(torch, dtype)).cuda()
+    got, want = torch.empty_like(b), torch.empty_like(b)
+    cfg = {"type": "ILU", "diagonalBased": dilu}
+    gb.Solver(A, cfg).solve(got, b)
+    gb.Solver(A, {**cfg, "kernel": "levels"}).solve(want, b)
+    assert not first_rows or not torch.isfinite(want).all()
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+    assert torch.equal(got.nan_to_num(1.5), want.nan_to_num(1.5))
