@@ -674,8 +674,7 @@ class PbicgstabNode : public Node {
     }
     if (mixed_) launchConvert(xw(), W, x, Wx, static_cast<int>(A_.n), s());  // exact: x holds float values
     else GR_CUDA(cudaMemcpyAsync(x, xw(), vb, cudaMemcpyDeviceToDevice, s()));
-    GR_CUDA(cudaStreamSynchronize(s()));
-    gr_stats out = stats();
+    gr_stats out = stats();  // x follows in stream order; the tree waits for it
     if (*errHost() != 0) {  // a device-side wait ran out (or an injected status)
       out.status = *errHost();
       out.converged = 0;
@@ -937,8 +936,7 @@ class MpirNode : public Node {
         printStats(cfg_, A_, st);
       }
     }
-    launchCastDown(phi_.get(), static_cast<float*>(x), E_, n, s());
-    GR_CUDA(cudaStreamSynchronize(s()));
+    launchCastDown(phi_.get(), static_cast<float*>(x), E_, n, s());  // the tree waits for it
     st.converged = conv;
     st.inner_iterations = innerTotal;
     if (cfg_.printPerformanceAfterSolve) printStats(cfg_, A_, st);
@@ -1109,6 +1107,7 @@ class Tree : public SolverTree {
     root_ = makeNode(A, *cfg_);
     GR_CUDA(cudaEventCreate(&e0_));
     GR_CUDA(cudaEventCreate(&e1_));
+    err_ = static_cast<int*>(acquirePinnedSlot());
   }
   ~Tree() override {
     // The nodes' buffers are released after this body: no work using them
@@ -1116,6 +1115,7 @@ class Tree : public SolverTree {
     cudaStreamSynchronize(A_.stream);
     cudaEventDestroy(e0_);
     cudaEventDestroy(e1_);
+    releasePinnedSlot(err_);
   }
   gr_stats solve(void* x, DType xt, const void* b, DType bt) override {
     if (xt != bt) fail(GR_EINVAL, "x and b must have the same type");
@@ -1123,14 +1123,14 @@ class Tree : public SolverTree {
     GR_CUDA(cudaEventRecord(e0_, A_.stream));
     gr_stats st = root_->solve(x, b, xt, nullptr);
     GR_CUDA(cudaEventRecord(e1_, A_.stream));
-    GR_CUDA(cudaEventSynchronize(e1_));
+    // A bounded device-side wait that ran out marks the solve as failed. The
+    // error word rides along to pinned memory, so that the host waits once.
+    GR_CUDA(cudaMemcpyAsync(err_, A_.errFlag.get(), sizeof(int), cudaMemcpyDeviceToHost, A_.stream));
+    GR_CUDA(cudaStreamSynchronize(A_.stream));
     float ms = 0;
     GR_CUDA(cudaEventElapsedTime(&ms, e0_, e1_));
     st.solve_ms = ms;
-    // A bounded device-side wait that ran out marks the solve as failed.
-    int err = 0;
-    GR_CUDA(cudaMemcpyAsync(&err, A_.errFlag.get(), sizeof(int), cudaMemcpyDeviceToHost, A_.stream));
-    GR_CUDA(cudaStreamSynchronize(A_.stream));
+    const int err = *err_;
     if (err != 0) {
       GR_CUDA(cudaMemsetAsync(A_.errFlag.get(), 0, sizeof(int), A_.stream));
       st.status = err;
@@ -1189,6 +1189,7 @@ class Tree : public SolverTree {
   std::unique_ptr<SolverConfig> cfg_;
   std::unique_ptr<Node> root_;
   cudaEvent_t e0_ = nullptr, e1_ = nullptr;
+  int* err_ = nullptr;  // pinned
 };
 
 }  // namespace
