@@ -82,7 +82,7 @@ void printStats(const SolverConfig& c, const DeviceMatrix& A, const gr_stats& st
 // Double: 128^3 / 1024 66.9 -> 49.3, 96^3 / 432 37.0 -> 32.8.
 // When the tiles need clearly more than one wave, float tiles break even
 // (192^3 / 2368: 104.3 -> 103.0; MPIR there 139.3 -> 134.7 ms) and double ones
-// stay on the level ring (172.1 us against 188.4 at best).
+// stay on the level ring (172.5 us against 181.0 at best).
 // Gauss-Seidel (two sweeps; a row costs a division and up to six entries, so
 // float tiles take two warps from 45 rows a level on; double tiles, of which
 // fewer fit an SM, one: the mesh with two 82.9): float 128^3 / 1024 tiles 77.9 -> 66.5,
