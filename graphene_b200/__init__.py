@@ -439,6 +439,12 @@ class Solver:
         check(_lib.lib().gr_solver_name(self._s, buf, 256))
         return buf.value.decode()
 
+    def sweepKernel(self, t: int = FLOAT32) -> str:
+        """The kernel of the ILU / Gauss-Seidel sweeps over vectors of type t (gr_solver_sweep_kernel)."""
+        buf = C.create_string_buffer(256)
+        check(_lib.lib().gr_solver_sweep_kernel(self._s, t, buf, 256))
+        return buf.value.decode()
+
     def solve(self, x, b) -> SolverStats:
         """x (in/out) and b: device tensors in tile order."""
         st = _lib.Stats()

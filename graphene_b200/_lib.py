@@ -108,6 +108,7 @@ SIGNATURES = {
     "gr_host_matrix_check_ilu_stream": (C.c_int, [vp, C.c_int, C.c_int, P(i32), P(i64)]),
     "gr_host_matrix_load_vector_mm": (C.c_int, [vp, C.c_char_p, C.c_int, vp]),
     "gr_host_matrix_check_ilu_ring": (C.c_int, [vp, C.c_int, C.c_int, i64, i32, i32, P(i64), P(i64), P(i32)]),
+    "gr_host_matrix_direct_shape": (C.c_int, [vp, i32, C.c_int, C.c_int, i32, i64, P(i32), P(i32)]),
     "gr_host_matrix_check_direct": (C.c_int, [vp, i32, C.c_int, i32, P(i32), P(i32), P(i32)]),
     "gr_host_matrix_check_gs_ring": (C.c_int, [vp, C.c_int, C.c_int, i64, i32, P(i64), P(i64), P(i32), P(i32)]),
     "gr_host_matrix_set_spmv_layout": (C.c_int, [vp, i32]),
@@ -152,6 +153,7 @@ SIGNATURES = {
     "gr_solve_host": (C.c_int, [vp, vp, C.c_int, vp, C.c_int, P(Stats)]),
     "gr_solver_phi": (C.c_int, [vp, vp, C.c_int]),
     "gr_solver_name": (C.c_int, [vp, C.c_char_p, C.c_size_t]),
+    "gr_solver_sweep_kernel": (C.c_int, [vp, C.c_int, C.c_char_p, C.c_size_t]),
     "gr_config_parse": (C.c_int, [C.c_char_p, C.c_char_p, C.c_size_t, C.c_char_p, C.c_size_t]),
 }
 

@@ -417,6 +417,19 @@ int gr_host_matrix_check_direct(const gr_host_matrix* h, int32_t sweep, int dilu
   });
 }
 
+int gr_host_matrix_direct_shape(const gr_host_matrix* h, int32_t sweep, gr_dtype coefficients, gr_dtype vectors,
+                                int32_t num_sms, int64_t smem_per_sm, int32_t* warps, int32_t* depth) {
+  return guarded([&] {
+    need(h, "matrix");
+    if (sweep < 0 || sweep > 1) gr::fail(GR_EINVAL, "sweep must be 0 (ILU) or 1 (Gauss-Seidel)");
+    if (num_sms < 1 || smem_per_sm < 1) gr::fail(GR_EINVAL, "num_sms and smem_per_sm must be positive");
+    const gr::DirectShape d = gr::directShape(*h->m, sweep == 0 ? gr::RingKind::Ilu : gr::RingKind::GaussSeidel,
+                                              gr::toDType(coefficients), gr::toDType(vectors), num_sms, smem_per_sm);
+    if (warps) *warps = d.warps;
+    if (depth) *depth = d.depth;
+  });
+}
+
 int gr_host_matrix_set_spmv_layout(gr_host_matrix* h, int32_t layout) {
   return guarded([&] {
     need(h, "matrix");
@@ -701,6 +714,17 @@ int gr_solver_name(const gr_solver* s, char* buf, size_t len) {
     std::string nm = s->s->name();
     if (len == 0) gr::fail(GR_EINVAL, "buffer length is 0");
     std::strncpy(buf, nm.c_str(), len - 1);
+    buf[len - 1] = '\0';
+  });
+}
+
+int gr_solver_sweep_kernel(const gr_solver* s, gr_dtype vectors, char* buf, size_t len) {
+  return guarded([&] {
+    need(s, "solver");
+    need(buf, "buf");
+    if (len == 0) gr::fail(GR_EINVAL, "buffer length is 0");
+    const std::string k = s->s->sweepKernel(gr::toDType(vectors));
+    std::strncpy(buf, k.c_str(), len - 1);
     buf[len - 1] = '\0';
   });
 }

@@ -41,7 +41,7 @@ struct SolverConfig {
   MultiColorMode factorizeMulticolor = MultiColorMode::Auto;
   bool diagonalBased = false;
   // Extension: substitution kernel, "auto" (the direct record kernel where
-  // directShape, solvers.cu, has it faster, else the host-scheduled ring kernel
+  // directShape, direct.cpp, has it faster, else the host-scheduled ring kernel
   // when a tile fits shared memory, else the level-schedule kernel; an option
   // of the ring kernel selects that one), "ring",
   // "tma" (chunked byte ring with a producer warp), "warp" (warp per tile)
@@ -107,7 +107,7 @@ struct SolverConfig {
   // computes them (float32 vectors only).
   bool reduceRef = false;
   // Gauss-Seidel sweep kernel: 0 auto (the direct record kernel where
-  // directShape, solvers.cu, has it faster; else the level ring with one warp
+  // directShape, direct.cpp, has it faster; else the level ring with one warp
   // per tile for float coefficients when a tile fits shared memory, a block
   // per tile for double coefficients and in batches), 1
   // the level ring with a block per tile, 2 level schedules in global

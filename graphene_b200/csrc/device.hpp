@@ -419,12 +419,25 @@ struct DirectPlan {
   RingKind kind = RingKind::Ilu;
   bool dilu = false, second = false, gsInPlace = false;
   bool longForward = false;  // ILU: the forward sweep has rows of more than three entries
-  i32 warps = 1, depth = 8, maxSteps = 0;  // depth: steps copied ahead
+  i32 warps = 1, maxSteps = 0;
   i64 records = 0, units = 0, maxRows = 0, maxXSlots = 0;
   bool factors = false;
   DBuf levelStart, levels, transposed, transposed2;
   DBuf src, src2, tail, tail2, steps, stepStart, stepRecord, stepUnit, haloStart, haloSrc;
 };
+// Shared memory of a block that copies `depth` steps ahead over vectors of
+// type W: places, x (Gauss-Seidel: and the right-hand side) and the step
+// table.
+size_t directSmem(const DirectPlan& P, DType coefficients, DType W, i32 depth);
+// Warps a tile and steps copied ahead of the direct sweep kernels; warps 0:
+// another kernel is the better choice.
+struct DirectShape {
+  i32 warps = 0, depth = 0;
+};
+constexpr i32 kDirectGsDepth = 4;  // Gauss-Seidel sweeps are built for this depth only
+// The choice for vectors of type `vec` on a device with numSMs SMs of
+// smemPerSM bytes of shared memory (rule and figures: direct.cpp).
+DirectShape directShape(const HostMatrix& H, RingKind kind, DType coefficients, DType vec, i32 numSMs, i64 smemPerSM);
 
 // Kinds of entries a schedule keeps per row.
 enum class SweepEntries {
@@ -491,9 +504,9 @@ struct DeviceMatrix {
   LevelRing& levelRing(bool dilu, i64 ringBytes, i32 group, bool allowCompact = true,
                        RingKind kind = RingKind::Ilu, bool records = false);
 
-  std::map<std::tuple<int, bool, i32, i32>, std::unique_ptr<DirectPlan>> directPlans;  // [(kind, dilu, warps, depth)]
+  std::map<std::tuple<int, bool, i32>, std::unique_ptr<DirectPlan>> directPlans;  // [(kind, dilu, warps)]
   // nullptr when the direct kernels cannot run this sweep.
-  DirectPlan* directPlan(RingKind kind, bool dilu, i32 warps, i32 depth);
+  DirectPlan* directPlan(RingKind kind, bool dilu, i32 warps);
 
   // Device error word written by kernels whose bounded waits ran out
   // (GR_ETIMEOUT); 0 when clean.

@@ -419,8 +419,116 @@ void checkDirect(const HostMatrix& H, const HostDirect& D) {
   });
 }
 
-DirectPlan* DeviceMatrix::directPlan(RingKind kind, bool dilu, i32 warps, i32 depth) {
-  auto key = std::make_tuple(static_cast<int>(kind), dilu, warps, depth);
+size_t directSmem(const DirectPlan& P, DType coefficients, DType W, i32 depth) {
+  const size_t rec = coefficients == DType::F32 ? (P.second ? 44 : 24) : (P.second ? 72 : 40);
+  const i64 rhs = P.kind == RingKind::Ilu ? 0 : (P.maxRows + 3) / 4 * 4;
+  return rec * static_cast<size_t>(depth) * 32 * static_cast<size_t>(P.warps) +
+         static_cast<size_t>((P.maxXSlots + 3) / 4 * 4 + rhs) * dtypeSize(W) + 4 * static_cast<size_t>(P.maxSteps);
+}
+
+// What counts is how many tiles share an SM (t), how many rows a level has,
+// how many tiles are resident at once, and whether the sweep's data stay in
+// L2; results do not depend on the shape. All figures: us on B200, level ring
+// -> direct, back-to-back applications; e/P: e^3 grid in P tiles, m: the
+// permuted hexahedral mesh.
+//
+// ILU, float vectors. Warps: with t <= 1 a wide level needs four (64/64, 89
+// rows a level: 37.0 -> 18.6, two 20.7), a narrow one two (32/64, 23 rows:
+// 16.5 -> 8.4). Up to two tiles an SM, four from 80 rows a level on (128/296:
+// 65.6 -> 43.2, two 47.4; below, 96/300: 39.6 -> 28.0, four 31.9). Then two
+// while a level fills them (128/512, 89 rows: 46.3 -> 39.1; 160/600, 119 rows:
+// 118.9 -> 100.1, one 108.7), else one (64/512: 18.6 -> 10.4; 128/1024: 41.2 ->
+// 35.0, two 41.0). Depth: 8, or 4 where only then all tiles are resident
+// (160/1370: 91.7 -> 80.0, with 8 103.7). A last wave that is not full costs
+// more than it does the ring, whose blocks hold less: ring from 1.3 waves on
+// (192/1184, 1.6: 125.9, direct 148; 176/2000, 1.5: 98.8, 108.3; 176/4096,
+// 2.3: 90, 105), for levels of 25 to 40 rows from two on (140x151x174/4944,
+// 2.4: 74.0, 78.9; 176x176x130/6185, 3.0: 84.1, 90.7; 144/3000, 1.6: 73.8 ->
+// 63.9); with two full waves they break even (192/2368: 104.9, 104.8).
+// Narrower levels cost the ring its hand-overs and always run direct (2048^2
+// in 2368 tiles, 20 rows: 150.2 -> 91.5, a chain of 2^20 rows in 1024: 1154 ->
+// 207). Levels of a step of two warps and a little more, five or six tiles an
+// SM, data beyond L2: ring (144/800: 59.5, 69.7; 128/700: 49.0, 51.4; the same
+// in L2, m100/700: 30.8 -> 22.7).
+//
+// ILU, double vectors. A step costs twice the cycles, so that few resident
+// warps no longer hide DRAM. Float coefficients: ring beyond about 165 MB
+// (160/600: 151.6, direct 160.7; 160/1370: 138.3, 154; 144/1300: 89.9, 110;
+// below 128/1024: 66.4 -> 46.9), for levels of 25 to 40 rows from 2.1 waves on
+// (160/4096: 91, 100; 144/3000: 114 -> 87); beyond half of L2 for wide levels
+// on up to 2.5 tiles an SM (128/148: 107.5, 125; 112/300: 73.5, 89; 96/148:
+// 51.4 -> 43) and on little more than four (130x107x112/609: 51.2, 59.5;
+// 112/750: 45.1, 45.3). Double coefficients: ring for more than one and a
+// quarter waves, for up to four tiles an SM (wide levels: five) beyond L2
+// (128/148: 105.5, 125; 112/300: 73.9, 95; 112/450: 47.3, 52.1; 120/640: 53.4,
+// 59.9; 128/512: 57.4, 56.3; below, 96/148: 49.3 -> 43.3) and from three on
+// already in L2 (96/560: 32.9, 35.0; m100/700: 32.8, 37.0); else direct
+// (128/1024: 67.0 -> 49.2, 96/1200: 47.3 -> 33.5).
+//
+// Gauss-Seidel (two sweeps; a row costs a division and up to six entries).
+// Float coefficients: direct always; four warps with t <= 2, two from 45 rows
+// a level on (128/1024: 78.0 -> 65.9, 160/1370: 264.5 -> 153.6, m100/1024:
+// 49.4 -> 40.8, 192/1184 with double vectors: 1591 -> 1145). Double
+// coefficients, whose divisions keep the ring's warps as busy: direct with
+// t > 4 in one wave (one warp; m100/1024: 86.2 -> 62, 64/1000: 49.3 -> 33.0;
+// 109x80x107/931, 1.05 waves: 82, 107) and on few tiles of very wide levels
+// (four warps; m100/256, 202 rows: 97 -> 64, m80/148: 49.3 -> 45.2). Between,
+// the ring: 96/432: 61.4, direct 82; 112/450: 127, 242; m80/400: 37.1, 53;
+// 80/256: 49.9, 57.
+DirectShape directShape(const HostMatrix& H, RingKind kind, DType coefficients, DType vec, i32 numSMs,
+                        i64 smemPerSM) {
+  const bool gs = kind != RingKind::Ilu, f32 = coefficients == DType::F32;
+  i64 levels = 1, halo = 0;
+  for (i32 T = 0; T < H.P; ++T) {
+    levels += H.nLowerLevels[T];
+    halo = std::max(halo, H.tiles[T].nHalo);
+  }
+  const double t = static_cast<double>(H.P) / numSMs, rows = static_cast<double>(H.n) / static_cast<double>(levels);
+  // Waves of blocks with room for second triples, copying d steps ahead.
+  const i64 vs = static_cast<i64>(dtypeSize(vec)), rec = f32 ? 44 : 72;
+  auto waves = [&](i32 warps, i32 d) {
+    i64 steps = 0;  // of the longest tile, at most
+    for (i32 T = 0; T < H.P; ++T) {
+      const i64 nRows = H.tileStart[T + 1] - H.tileStart[T];
+      steps = std::max(steps, H.nLowerLevels[T] + (gs ? 0 : H.nUpperLevels[T]) + (gs ? 1 : 2) * (nRows / (32 * warps)));
+    }
+    const i64 block = vs * (gs ? 2 * H.maxTileRows + halo : H.maxTileRows) + rec * d * 32 * warps +
+                      4 * (steps + kDirectHead + kDirectAhead) + 1024;
+    const i64 slots = smemPerSM / block * numSMs;
+    return slots > 0 ? static_cast<double>(H.P) / static_cast<double>(slots) : 1e9;
+  };
+  if (gs) {
+    i32 warps = t <= 2 ? 4 : rows > 45 ? 2 : 1;
+    if (!f32) {
+      warps = t <= 2 && rows > 150 ? 4 : t > 4 ? 1 : 0;
+      if (warps == 0 || waves(warps, kDirectGsDepth) > 1) return {};
+    }
+    return {warps, kDirectGsDepth};
+  }
+  const i32 warps = t <= 1   ? (rows > 40 ? 4 : 2)
+                    : t <= 2 ? (rows > 80 ? 4 : 2)
+                    : t <= 4 ? (rows > 40 ? 2 : 1)
+                             : (t <= 6 && rows > 64 ? 2 : 1);
+  const i32 depth = waves(warps, 8) > 1 && waves(warps, 4) <= 1 ? 4 : 8;
+  const double w = waves(warps, depth);
+  // A seven-point grid's coefficients and two vectors.
+  const double mb = static_cast<double>(H.n) * (f32 ? 50 + 2 * vs : 116) * 1e-6;
+  bool ring;
+  if (!f32) {
+    ring = w > 1.25 || (rows > 40 && t <= (rows > 64 ? 5 : 4) && (mb > 120 || t > 3));
+  } else if (vec == DType::F64) {
+    ring = (mb > 165 && (rows > 40 || (rows > 25 && w > 2.1))) ||
+           (mb > 66 && ((rows > 80 && t <= 2.5) || (rows > 55 && t > 4 && t <= 5)));
+  } else {
+    ring = ((w < 1.96 || w > 2.02) && ((rows > 40 && w > 1.3) || (rows > 25 && w > 2))) ||
+           (mb > 100 && rows > 64 && rows < 90 && t > 4.5 && t <= 6);
+  }
+  if (ring) return {};
+  return {warps, depth};
+}
+
+DirectPlan* DeviceMatrix::directPlan(RingKind kind, bool dilu, i32 warps) {
+  auto key = std::make_tuple(static_cast<int>(kind), dilu, warps);
   auto it = directPlans.find(key);
   if (it != directPlans.end()) return it->second.get();
   std::unique_ptr<DirectPlan> R;
@@ -433,7 +541,6 @@ DirectPlan* DeviceMatrix::directPlan(RingKind kind, bool dilu, i32 warps, i32 de
     R->longForward = D.longForward;
     R->gsInPlace = D.gsInPlace;
     R->warps = warps;
-    R->depth = depth;
     R->maxSteps = D.maxSteps;
     R->records = D.records;
     R->units = D.units;

@@ -823,13 +823,6 @@ dev::DirectView directView(const DeviceMatrix& A, const DirectPlan& P, const DBu
                          P.longForward};
 }
 
-// Places, x (`extra` more slots) and the step table.
-size_t directSmem(const DirectPlan& P, DType vt, i64 extra, DType W) {
-  const size_t rec = vt == DType::F32 ? (P.second ? 44 : 24) : (P.second ? 72 : 40);
-  return rec * P.depth * 32 * static_cast<size_t>(P.warps) +
-         static_cast<size_t>((P.maxXSlots + 3) / 4 * 4 + extra) * dtypeSize(W) + 4 * static_cast<size_t>(P.maxSteps);
-}
-
 bool aligned16(std::initializer_list<const void*> ps) {
   uintptr_t bits = 0;
   for (const void* p : ps) bits |= reinterpret_cast<uintptr_t>(p);
@@ -838,11 +831,7 @@ bool aligned16(std::initializer_list<const void*> ps) {
 
 }  // namespace
 
-size_t iluDirectSmem(const DirectPlan& P, DType vt, DType W) { return directSmem(P, vt, 0, W); }
-
 size_t directBytes(const DirectPlan& P) { return 16 * std::max<size_t>(1, static_cast<size_t>(P.units)); }
-
-size_t gsDirectSmem(const DirectPlan& P, DType vt, DType W) { return directSmem(P, vt, (P.maxRows + 3) / 4 * 4, W); }
 
 void launchDirectPack(DeviceMatrix& A, const DirectPlan& P, DBuf& data, const void* F, const void* inv,
                       cudaStream_t s) {
@@ -892,10 +881,10 @@ auto iluDirectFor(int warps) {
                       : dev::iluDirectKernel<MV, W, NT, 4, DEPTH, DILU>;
 }
 template <class MV, class W, int NT, bool DILU>
-void iluDirectT(DeviceMatrix& A, const DirectPlan& P, const DBuf& data, const PrologueArgs& p, void* y,
+void iluDirectT(DeviceMatrix& A, const DirectPlan& P, i32 depth, const DBuf& data, const PrologueArgs& p, void* y,
                 cudaStream_t s) {
-  const size_t smem = iluDirectSmem(P, dtypeOf<MV>(), dtypeOf<W>());
-  auto kernel = P.depth == 4 ? iluDirectFor<MV, W, NT, DILU, 4>(P.warps) : iluDirectFor<MV, W, NT, DILU, 8>(P.warps);
+  const size_t smem = directSmem(P, dtypeOf<MV>(), dtypeOf<W>(), depth);
+  auto kernel = depth == 4 ? iluDirectFor<MV, W, NT, DILU, 4>(P.warps) : iluDirectFor<MV, W, NT, DILU, 8>(P.warps);
   ensureDynamicSmem(reinterpret_cast<const void*>(kernel), smem);
   preferSharedCarveout(reinterpret_cast<const void*>(kernel));
   dev::SPro<W> pro{static_cast<int>(p.kind), static_cast<const W*>(p.b), static_cast<const W*>(p.r),
@@ -906,17 +895,18 @@ void iluDirectT(DeviceMatrix& A, const DirectPlan& P, const DBuf& data, const Pr
 }
 }  // namespace
 
-void launchIluDirect(DeviceMatrix& A, const DirectPlan& P, const DBuf& data, bool dilu, const PrologueArgs& pro,
-                     void* y, DType W, cudaStream_t s) {
+void launchIluDirect(DeviceMatrix& A, const DirectPlan& P, i32 depth, const DBuf& data, bool dilu,
+                     const PrologueArgs& pro, void* y, DType W, cudaStream_t s) {
+  if (depth != 4 && depth != 8) fail(GR_EINVAL, "direct sweeps copy 4 or 8 steps ahead");
   auto go = [&](auto mv, auto w) {
     using MV = decltype(mv);
     using Wt = decltype(w);
     if (P.second) {
-      if (dilu) iluDirectT<MV, Wt, 2, true>(A, P, data, pro, y, s);
-      else iluDirectT<MV, Wt, 2, false>(A, P, data, pro, y, s);
+      if (dilu) iluDirectT<MV, Wt, 2, true>(A, P, depth, data, pro, y, s);
+      else iluDirectT<MV, Wt, 2, false>(A, P, depth, data, pro, y, s);
     } else {
-      if (dilu) iluDirectT<MV, Wt, 1, true>(A, P, data, pro, y, s);
-      else iluDirectT<MV, Wt, 1, false>(A, P, data, pro, y, s);
+      if (dilu) iluDirectT<MV, Wt, 1, true>(A, P, depth, data, pro, y, s);
+      else iluDirectT<MV, Wt, 1, false>(A, P, depth, data, pro, y, s);
     }
   };
   if (A.vt == DType::F32 && W == DType::F32) go(0.0f, 0.0f);
@@ -926,17 +916,17 @@ void launchIluDirect(DeviceMatrix& A, const DirectPlan& P, const DBuf& data, boo
 }
 
 namespace {
-template <class MV, class X, class W, int NT, int DEPTH>
+template <class MV, class X, class W, int NT>
 auto gsDirectFor(int warps) {
-  return warps == 1   ? dev::gsDirectKernel<MV, X, W, NT, 1, DEPTH>
-         : warps == 2 ? dev::gsDirectKernel<MV, X, W, NT, 2, DEPTH>
-                      : dev::gsDirectKernel<MV, X, W, NT, 4, DEPTH>;
+  return warps == 1   ? dev::gsDirectKernel<MV, X, W, NT, 1, kDirectGsDepth>
+         : warps == 2 ? dev::gsDirectKernel<MV, X, W, NT, 2, kDirectGsDepth>
+                      : dev::gsDirectKernel<MV, X, W, NT, 4, kDirectGsDepth>;
 }
 template <class MV, class X, class W, int NT>
 void gsDirectT(DeviceMatrix& A, const DirectPlan& P, const DBuf& data, const PrologueArgs& p, bool seedB,
                const void* xin, bool xinZero, void* xout, cudaStream_t s, bool dropHalo) {
-  const size_t smem = gsDirectSmem(P, dtypeOf<MV>(), dtypeOf<W>());
-  auto kernel = P.depth == 4 ? gsDirectFor<MV, X, W, NT, 4>(P.warps) : gsDirectFor<MV, X, W, NT, 8>(P.warps);
+  const size_t smem = directSmem(P, dtypeOf<MV>(), dtypeOf<W>(), kDirectGsDepth);
+  auto kernel = gsDirectFor<MV, X, W, NT>(P.warps);
   ensureDynamicSmem(reinterpret_cast<const void*>(kernel), smem);
   preferSharedCarveout(reinterpret_cast<const void*>(kernel));
   dev::SPro<X> pro{static_cast<int>(p.kind), static_cast<const X*>(p.b), static_cast<const X*>(p.r),

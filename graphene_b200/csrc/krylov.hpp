@@ -102,12 +102,9 @@ void launchIluWarpRing(DeviceMatrix& A, const LevelRing& R, const void* stream, 
 void launchIluRing(DeviceMatrix& A, const LevelRing& R, const void* stream, bool dilu, const PrologueArgs& pro,
                    void* y, DType W, int l2Ahead, bool unroll, cudaStream_t s, bool pairRows = false, int computeWarps = 0,
                    bool waiter = true, bool producer = true);
-// Direct sweeps (kernels_direct.cu): shared memory of a block for vectors of
-// type W, the bytes of a solver's blocks (with what the kernels prefetch
-// beyond the last), their packing, and the
-// launches (launchGsDirect: the arguments of launchGsRing below).
-size_t iluDirectSmem(const DirectPlan& P, DType vt, DType W);
-size_t gsDirectSmem(const DirectPlan& P, DType vt, DType W);
+// Direct sweeps (kernels_direct.cu): the bytes of a solver's blocks, their
+// packing, and the launches (depth: steps copied ahead; launchGsDirect: the
+// arguments of launchGsRing below).
 size_t directBytes(const DirectPlan& P);
 void launchDirectPack(DeviceMatrix& A, const DirectPlan& P, DBuf& data, const void* F, const void* inv,
                       cudaStream_t s);
@@ -115,8 +112,8 @@ void launchDirectPack(DeviceMatrix& A, const DirectPlan& P, DBuf& data, const vo
 // with `factors`), and its shared memory.
 size_t directFactorSmem(const DirectPlan& P, DType vt);
 void launchIluFactorDirect(DeviceMatrix& A, const DirectPlan& P, DBuf& data, bool dilu, cudaStream_t s);
-void launchIluDirect(DeviceMatrix& A, const DirectPlan& P, const DBuf& data, bool dilu, const PrologueArgs& pro,
-                     void* y, DType W, cudaStream_t s);
+void launchIluDirect(DeviceMatrix& A, const DirectPlan& P, i32 depth, const DBuf& data, bool dilu,
+                     const PrologueArgs& pro, void* y, DType W, cudaStream_t s);
 void launchGsDirect(DeviceMatrix& A, const DirectPlan& P, const DBuf& data, const PrologueArgs& pro, bool seedB,
                     const void* xin, bool xinZero, void* xout, DType X, DType W, cudaStream_t s,
                     bool dropHalo = false);

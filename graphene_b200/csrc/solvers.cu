@@ -8,6 +8,7 @@
 //   MpirNode         iterativerefinement::Solver (iterative-refinement/Solver.cpp:48-128)
 //   RestarterNode    restarter::Solver        (restarter/Solver.cpp:34-56)
 // and Solver::createSolver's dispatch is makeNode (Solver.cpp:32-56).
+#include <array>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -38,6 +39,9 @@ class Node {
   virtual void prepare(DType) {}
   // Recomputes the parts that depend on the matrix's values, in place.
   virtual void refresh() {}
+  // The kernel of this solver's sweeps (its preconditioner's) over vectors of
+  // type W; empty when it has none.
+  virtual std::string sweepKernel(DType) const { return ""; }
   // Per-system statistics of the last solve of a batch.
   virtual std::vector<gr_stats> batchStats() const {
     fail(GR_EUNSUPPORTED, "only PBiCGStab and IterativeRefinement solve batches");
@@ -65,64 +69,21 @@ void printStats(const SolverConfig& c, const DeviceMatrix& A, const gr_stats& st
                st.iterations, st.converged ? "true" : "false", st.singular ? "true" : "false");
 }
 
-// Warps a tile and steps copied ahead of the direct sweep kernels
-// (kernels_direct.cu) for matrix A; {0, 0}: the level rings are the better
-// choice. What counts is how many tiles share an SM (t) and how many rows a
-// level has; results do not depend on the shape.
-//
-// ILU, float (us on B200, level ring -> direct; seven-point grids): with t <=
-// 1 a wide level needs the warps (64^3 / 64 tiles, 93 rows a level: 37.0 ->
-// 18.5 with four, 19.8 with two), a narrow one two (32^3 / 64 tiles, 23 rows:
-// 16.5 -> 8.2); between, two warps when a level fills them (128^3 / 512 tiles,
-// 93 rows: 45.5 -> 39.1; 96^3 / 432, 57 rows: 36.9 -> 22.6, with the records in
-// DRAM 44.2 -> 30.8, one warp 32.8), else one (64^3 / 512, 23 rows: 18.5 ->
-// 10.3); with t > 4 one warp, copying 8 steps
-// ahead where all tiles then fit the SMs at once (128^3 / 1024: 41.1 -> 34.9),
-// 4 where only then they do (160^3 / 1370: 90.8 -> 80.5, with 8 104.6).
-// Double: 128^3 / 1024 66.9 -> 49.3, 96^3 / 432 37.0 -> 32.8.
-// When the tiles need clearly more than one wave, float tiles break even
-// (192^3 / 2368: 104.3 -> 103.0; MPIR there 139.3 -> 134.7 ms) and double ones
-// stay on the level ring (172.5 us against 181.0 at best).
-// Gauss-Seidel (two sweeps; a row costs a division and up to six entries, so
-// float tiles take two warps from 45 rows a level on; double tiles, of which
-// fewer fit an SM, one: the mesh with two 82.9): float 128^3 / 1024 tiles 77.9 -> 66.5,
-// 160^3 / 1370 262.5 -> 156.6, 100^3 mesh / 1024 (36 rows) 49.2 -> 36.9, / 256
-// 82.0 -> 40.4; double mesh 86.0 -> 60.2 and 99.2 -> 63.2, but 128^3 / 1024
-// (1.7 waves) 155.6 -> 190.4.
-std::pair<i32, i32> directShape(const DeviceMatrix& A, RingKind kind) {
-  const HostMatrix& H = *A.host;
-  const bool gs = kind != RingKind::Ilu, f32 = A.vt == DType::F32;
-  i64 levels = 1, halo = 0;
-  for (i32 T = 0; T < H.P; ++T) {
-    levels += H.nLowerLevels[T];
-    halo = std::max(halo, H.tiles[T].nHalo);
-  }
-  const double t = static_cast<double>(H.P) / A.numSMs, rows = static_cast<double>(H.n) / static_cast<double>(levels);
-  i32 warps = 1, depth = gs ? 4 : 8;
-  if (gs) warps = t <= 2 ? 4 : f32 && rows > 45 ? 2 : 1;
-  else if (t <= 1) warps = rows > 40 ? 4 : 2;
-  else if (t <= 2) warps = 2;
-  else if (t <= 4) warps = rows > 40 ? 2 : 1;
-  // Whether all tiles are resident at once: the x slots (and the right-hand
-  // side), places for records with second triples, and about 2 KB of step
-  // table and reserve a block.
-  const i64 vs = f32 ? 4 : 8, rec = f32 ? 44 : 72;
-  const i64 fixed = vs * (gs ? 2 * H.maxTileRows + halo : H.maxTileRows) + 2048;
+DirectShape directShapeFor(const DeviceMatrix& A, RingKind kind, DType vec) {
   int perSM = 233472;
   GR_CUDA(cudaDeviceGetAttribute(&perSM, cudaDevAttrMaxSharedMemoryPerMultiprocessor, A.device));
-  auto waves = [&](i32 d) {
-    const i64 slots = perSM / (fixed + rec * d * 32 * warps) * A.numSMs;
-    return slots > 0 ? static_cast<double>(H.P) / static_cast<double>(slots) : 1e9;
-  };
-  if (depth == 8 && waves(8) > 1 && waves(4) <= 1) depth = 4;
-  if (!f32 && waves(depth) > 1.25) return {0, 0};
-  return {warps, depth};
+  return directShape(*A.host, kind, A.vt, vec, A.numSMs, perSM);
+}
+
+std::string directName(const DirectPlan& P, i32 depth) {
+  return "direct " + std::to_string(P.warps) + "x" + std::to_string(depth);
 }
 
 // ---------------------------------------------------------------------------
 class IluNode : public Node {
  public:
-  IluNode(DeviceMatrix& A, const SolverConfig& c) : Node(A, c), dilu_(c.diagonalBased) {
+  // direct false: without the direct kernels.
+  IluNode(DeviceMatrix& A, const SolverConfig& c, bool direct = true) : Node(A, c), dilu_(c.diagonalBased) {
     A.ensureLocalCrs();
     const size_t vs = dtypeSize(A.vt);
     // Streamed substitution when the ring and the tile slice fit in shared
@@ -140,12 +101,16 @@ class IluNode : public Node {
         fail(GR_EUNSUPPORTED, "the warp ring ILU kernel does not fit this matrix's tiles in shared memory");
       kernel_ = 5;
     }
-    if (c.iluKernel == 0 && !ringOptions(c)) {
-      const auto [warps, depth] = directShape(A, RingKind::Ilu);
-      DirectPlan* P = warps > 0 ? A.directPlan(RingKind::Ilu, dilu_, warps, depth) : nullptr;
-      if (P && iluDirectSmem(*P, A.vt, DType::F64) <= smemMax) {
+    if (direct && c.iluKernel == 0 && !ringOptions(c)) {
+      const DirectShape own = directShapeFor(A, RingKind::Ilu, A.vt);
+      const DirectShape wide = directShapeFor(A, RingKind::Ilu, DType::F64);
+      depth_ = own.depth;
+      wideDepth_ = wide.warps > 0 ? wide.depth : own.depth;
+      DirectPlan* P = own.warps > 0 ? A.directPlan(RingKind::Ilu, dilu_, own.warps) : nullptr;
+      if (P && directSmem(*P, A.vt, DType::F64, std::max(depth_, wideDepth_)) <= smemMax) {
         kernel_ = 6;
         direct_ = P;
+        wideOther_ = wide.warps == 0;
       }
     }
     if (kernel_ == 2 && (c.iluKernel == 0 || c.iluKernel == 4)) {
@@ -191,7 +156,27 @@ class IluNode : public Node {
     }
     factorAndPack();
   }
-  void refresh() override { factorAndPack(); }
+  void refresh() override {
+    factorAndPack();
+    if (wide_) wide_->refresh();
+  }
+  // Double vectors over float coefficients for which directShape has another
+  // kernel: a second solver of this preconditioner, made when the first such
+  // vectors come (its blocks cost as much memory and set-up as this one's).
+  void prepare(DType W) override {
+    if (W != DType::F64 || !wideOther_) return;
+    wideOther_ = false;
+    try {
+      wide_ = std::make_unique<IluNode>(A_, cfg_, false);
+    } catch (const Error&) {  // no room for it: the direct kernel serves both types
+    }
+    if (wide_ && wide_->kernel_ != 4) wide_.reset();  // likewise without the ring
+  }
+  std::string sweepKernel(DType W) const override {
+    if (kernel_ == 6 && W == DType::F64 && (wide_ || wideOther_)) return "ring";
+    if (kernel_ != 6) return std::array{"", "tma", "levels", "warp", "ring", "wring"}[kernel_];
+    return directName(*direct_, W == DType::F64 ? wideDepth_ : depth_) + (fusedFactor_ ? " factor" : "");
+  }
   // ilu::Solver::factorize (ilu/Solver.cpp:44-51, :134-292) of the matrix's
   // current values, and the packing of the factors into this solver's own
   // level blocks (the buffers allocated at construction).
@@ -233,14 +218,17 @@ class IluNode : public Node {
     pro.kind = Prologue::Plain;
     pro.b = b;
     pro.st = gate;
+    prepare(W);
     apply(pro, x, W);
     gr_stats st{};
     st.iterations = 1;  // ilu/Solver.cpp:571-573
     return st;
   }
   void apply(const PrologueArgs& pro, void* y, DType W) {
-    if (kernel_ == 6)
-      launchIluDirect(A_, *direct_, stream_, dilu_, pro, y, W, s());
+    if (wide_ && W == DType::F64)
+      wide_->apply(pro, y, W);
+    else if (kernel_ == 6)
+      launchIluDirect(A_, *direct_, W == DType::F64 ? wideDepth_ : depth_, stream_, dilu_, pro, y, W, s());
     else if (kernel_ == 5)
       launchIluWarpRing(A_, *ring_, stream_.get(), dilu_, pro, y, W, cfg_.warpsPerBlock, cfg_.pairRows, s());
     else if (kernel_ == 4)
@@ -302,6 +290,9 @@ class IluNode : public Node {
            c.pairRows || c.computeWarps != 0 || !c.waitingWarp || !c.producerWarp || c.unrollRows != -1;
   }
   const DirectPlan* direct_ = nullptr;
+  i32 depth_ = 0, wideDepth_ = 0;  // steps copied ahead: float, double vectors
+  bool wideOther_ = false;         // double vectors take wide_ (not made yet)
+  std::unique_ptr<IluNode> wide_;
   bool fusedFactor_ = false;  // factorises straight into the direct sweep's blocks
   // 1 tma ring, 2 level schedule, 3 warp per tile, 4 host-scheduled ring, 5 its warp-per-tile form, 6 direct records
   int kernel_ = 2;
@@ -320,11 +311,12 @@ class GsNode : public Node {
     // vector type): one ring with every entry, and one with the lower
     // entries only for sweeps that start from x = 0.
     if (c.gsKernel == 0 && c.ringRecords && c.warpsPerBlock == 1 && !c.gsPairRows) {
-      const auto [warps, depth] = directShape(A, RingKind::GaussSeidel);
-      DirectPlan* P = warps > 0 ? A.directPlan(RingKind::GaussSeidel, false, warps, depth) : nullptr;
-      DirectPlan* L = P ? A.directPlan(RingKind::GaussSeidelLower, false, warps, depth) : nullptr;
+      const i32 warps = directShapeFor(A, RingKind::GaussSeidel, A.vt).warps;
+      DirectPlan* P = warps > 0 ? A.directPlan(RingKind::GaussSeidel, false, warps) : nullptr;
+      DirectPlan* L = P ? A.directPlan(RingKind::GaussSeidelLower, false, warps) : nullptr;
       const size_t smemMax = static_cast<size_t>(maxDynamicSmem(A));
-      if (P && L && gsDirectSmem(*P, A.vt, DType::F64) <= smemMax && gsDirectSmem(*L, A.vt, DType::F64) <= smemMax) {
+      if (P && L && directSmem(*P, A.vt, DType::F64, kDirectGsDepth) <= smemMax &&
+          directSmem(*L, A.vt, DType::F64, kDirectGsDepth) <= smemMax) {
         direct_ = P;
         directLo_ = L;
       }
@@ -427,6 +419,9 @@ class GsNode : public Node {
   }
   bool usesInitialGuess() const override { return true; }
   void prepare(DType W) override { ensureTmp(W); }
+  std::string sweepKernel(DType) const override {
+    return direct_ ? directName(*direct_, kDirectGsDepth) : !ring_ ? "levels" : warpRing_ ? "wring" : "ring";
+  }
 
  private:
   gr_stats solveImpl(void* x, const void* b, DType W, const KState* gate, bool xZero) {
@@ -616,6 +611,7 @@ class PbicgstabNode : public Node {
       launchConvert(b, Wx, bw_.get(), W, static_cast<int>(A_.n), s());
     }
     const void* bW = mixed_ ? bw_.get() : b;
+    if (pre_) pre_->prepare(W);
     if (ref && refTiles_.bytes() < 2 * static_cast<size_t>(A_.P) * sizeof(float))
       refTiles_.alloc(2 * static_cast<size_t>(A_.P) * sizeof(float));
     const size_t vb = A_.n * dtypeSize(W);
@@ -686,6 +682,7 @@ class PbicgstabNode : public Node {
   void refresh() override {
     if (pre_) pre_->refresh();
   }
+  std::string sweepKernel(DType W) const override { return pre_ ? pre_->sweepKernel(workingType(cfg_, W)) : ""; }
   std::vector<gr_stats> batchStats() const override {
     std::vector<gr_stats> out(systems_);
     for (int k = 0; k < systems_; ++k) out[k] = statsOf(host_[k]);
@@ -944,6 +941,7 @@ class MpirNode : public Node {
   }
   bool usesInitialGuess() const override { return true; }
   void refresh() override { inner_->refresh(); }
+  std::string sweepKernel(DType W) const override { return inner_->sweepKernel(W); }
   void copyPhi(void* out, DType t) override {
     if (!phi_.get()) fail(GR_EINVAL, "no IterativeRefinement solve has run yet");
     launchConvert(phi_.get(), E_, out, t, A_.n, s());
@@ -1087,6 +1085,7 @@ class RestarterNode : public Node {
   bool usesInitialGuess() const override { return inner_->usesInitialGuess(); }
   void copyPhi(void* out, DType t) override { inner_->copyPhi(out, t); }
   void refresh() override { inner_->refresh(); }
+  std::string sweepKernel(DType W) const override { return inner_->sweepKernel(W); }
 
  private:
   std::unique_ptr<Node> inner_;
@@ -1179,6 +1178,7 @@ class Tree : public SolverTree {
   void copyPhi(void* out, DType t) override { root_->copyPhi(out, t); }
   std::vector<gr_stats> batchStats() const override { return root_->batchStats(); }
   std::string name() const override { return cfg_->solverName(); }
+  std::string sweepKernel(DType W) const override { return root_->sweepKernel(W); }
   void refresh() override {
     root_->refresh();
     GR_CUDA(cudaStreamSynchronize(A_.stream));

@@ -28,6 +28,8 @@ class SolverTree {
   // Per-system statistics of the last solve on a batch matrix.
   virtual std::vector<gr_stats> batchStats() const = 0;
   virtual std::string name() const = 0;
+  // The kernel of the tree's ILU or Gauss-Seidel sweeps over vectors of type W.
+  virtual std::string sweepKernel(DType W) const = 0;
   // After the matrix's values were replaced (DeviceMatrix::updateValues):
   // recomputes every value-dependent part (ILU factors, packed level
   // blocks) in the buffers the tree already owns, so its captured iteration

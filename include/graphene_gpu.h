@@ -309,6 +309,16 @@ int gr_host_matrix_check_gs_ring(const gr_host_matrix* h, int lower_only, gr_dty
 int gr_host_matrix_check_direct(const gr_host_matrix* h, int32_t sweep, int dilu, int32_t warps, int32_t* max_steps,
                                 int32_t* second, int32_t* in_place);
 
+/* The automatic choice between the direct sweep kernels and the others, for
+ * coefficients and vectors of the given types on a device of num_sms SMs with
+ * smem_per_sm bytes of shared memory each (B200: 148, 233472): the warps a
+ * tile and the steps copied ahead, or 0 and 0 for another kernel. sweep 0:
+ * ILU(0) / DILU, 1: Gauss-Seidel. The matrix must also pass
+ * gr_host_matrix_check_direct and fit a block's shared memory. Host only. No
+ * counterpart in the reference. */
+int gr_host_matrix_direct_shape(const gr_host_matrix* h, int32_t sweep, gr_dtype coefficients, gr_dtype vectors,
+                                int32_t num_sms, int64_t smem_per_sm, int32_t* warps, int32_t* depth);
+
 /* DistributedTileLayout::loadVectorFromFile (DistributedTileLayout.cpp:185-206,
  * without halo): reads a MatrixMarket vector (a "vector" object, coordinate
  * or array, or the first column of a "matrix" object; unlisted entries are
@@ -478,6 +488,13 @@ int gr_matrix_update_global_values(gr_matrix* A, const double* g_val, const doub
 
 /* Name of the solver tree, e.g. "IterativeRefinement(PBiCGStab(ILU(0)))". */
 int gr_solver_name(const gr_solver* s, char* buf, size_t len);
+/* The kernel that a solver's ILU or Gauss-Seidel sweeps (a Krylov solver's:
+ * its preconditioner's) run over vectors of the given type: "direct WxD" (W
+ * warps a tile, D steps copied ahead; " factor" follows when the
+ * factorisation writes the sweep's records itself), "ring", "wring", "tma",
+ * "warp" or "levels"; empty without such sweeps. No counterpart in the
+ * reference. */
+int gr_solver_sweep_kernel(const gr_solver* s, gr_dtype vectors, char* buf, size_t len);
 
 /* Parses a solver configuration without a matrix or a GPU
  * (Configuration::fromJSON, matrix/solver/Configuration.cpp:103-136) and

@@ -1,0 +1,106 @@
+"""The automatic choice between the direct sweeps and the other kernels
+(directShape, direct.cpp): the shape it gives for matrices on each side of its
+lines, and what solvers then run."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import graphene_b200 as gb
+
+ILU, GS = 0, 1
+F32, F64 = gb.FLOAT32, gb.FLOAT64
+B200 = (148, 233472)
+
+
+def shape(h, sweep, coef, vec, sms=B200[0]):
+    w, d = C.c_int32(), C.c_int32()
+    gb._lib.check(gb._lib.lib().gr_host_matrix_direct_shape(h._h, sweep, coef, vec, sms, B200[1], C.byref(w),
+                                                            C.byref(d)))
+    return w.value, d.value
+
+
+def grid(n, tiles):
+    return gb.generate3DPoissonMatrix(F32, n, n, n, tiles, gb.PART_RCB)
+
+
+def mesh(n, tiles):
+    return gb.generateLduMesh(n, n, n, numTiles=tiles, partitioner=gb.PART_RCB)
+
+
+# Where the level rings measured faster (figures at directShape) they are
+# taken: (matrix, sweep, coefficients, vectors).
+@pytest.mark.parametrize("make,sweep,coef,vec", [
+    (lambda: grid(96, 432), GS, F64, F64),
+    (lambda: grid(80, 400), GS, F64, F64),
+    (lambda: grid(80, 256), GS, F64, F64),
+    (lambda: mesh(80, 400), GS, F64, F64),
+    (lambda: mesh(40, 64), GS, F64, F64),
+    (lambda: gb.generate3DPoissonMatrix(F32, 109, 80, 107, 931, gb.PART_RCB), GS, F64, F64),
+    (lambda: grid(96, 560), ILU, F64, F64),
+    (lambda: grid(112, 300), ILU, F64, F64),
+    (lambda: grid(112, 300), ILU, F32, F64),
+])
+def test_ring_where_it_is_faster(make, sweep, coef, vec):
+    assert shape(make(), sweep, coef, vec) == (0, 0)
+
+
+@pytest.mark.parametrize("make,sweep,coef,vec,want", [
+    (lambda: grid(32, 64), ILU, F32, F32, (2, 8)),
+    (lambda: grid(64, 64), ILU, F32, F32, (4, 8)),
+    (lambda: grid(64, 64), ILU, F32, F64, (4, 8)),
+    (lambda: grid(64, 512), ILU, F32, F32, (1, 8)),
+    (lambda: grid(112, 300), ILU, F32, F32, (2, 8)),
+    (lambda: mesh(80, 256), ILU, F64, F64, (4, 8)),
+    (lambda: grid(96, 148), ILU, F64, F64, (4, 8)),
+    (lambda: grid(96, 1200), ILU, F64, F64, (1, 4)),
+    (lambda: grid(64, 64), GS, F32, F32, (4, 4)),
+    (lambda: grid(96, 432), GS, F32, F64, (2, 4)),
+    (lambda: grid(64, 512), GS, F32, F32, (1, 4)),
+    (lambda: grid(64, 1000), GS, F64, F64, (1, 4)),
+    (lambda: mesh(60, 64), GS, F64, F64, (4, 4)),
+    (lambda: mesh(100, 1024), GS, F64, F64, (1, 4)),
+])
+def test_direct_where_it_is_faster(make, sweep, coef, vec, want):
+    assert shape(make(), sweep, coef, vec) == want
+
+
+def test_last_wave():
+    """Float tiles in one and a half waves take the ring, in less or nearly two
+    the direct kernel, with four steps ahead where that makes one wave of more."""
+    h = grid(96, 592)  # 11 tiles an SM with 8 steps ahead, 15 with 4
+    got = {sms: shape(h, ILU, F32, F32, sms) for sms in (54, 45, 36, 27)}
+    assert got == {54: (1, 8), 45: (1, 4), 36: (0, 0), 27: (1, 8)}
+
+
+@pytest.mark.gpu
+def test_double_vectors_over_float_coefficients():
+    """One solver, float vectors through the direct kernel and double ones
+    through the ring: both as the level schedules, also after new values and
+    within PBiCGStab's captured iterations."""
+    import torch
+    h = grid(112, 300)
+    A = h.copyToTile()
+    s, p = gb.Solver(A, {"type": "ILU"}), gb.Solver(A, {"type": "PBiCGStab", "maxIterations": 4,
+                                                      "preconditioner": {"type": "ILU"}})
+    assert s.sweepKernel(F32) == "direct 2x8 factor" and s.sweepKernel(F64) == "ring"
+    assert p.sweepKernel(F64) == "ring"
+    g = torch.Generator().manual_seed(7)
+    b = torch.rand(h.numRows, generator=g, dtype=torch.float64).mul(2).sub(1).cuda()
+    rp, col, off, dg = h.globalCrs()
+    for scale in (1.0, 1.25):
+        A.updateGlobalValues(off * scale, dg)
+        s.refresh()
+        p.refresh()
+        for dt in (torch.float64, torch.float32, torch.float64):
+            want, got = (torch.zeros(h.numRows, dtype=dt, device="cuda") for _ in range(2))
+            gb.Solver(A, {"type": "ILU", "kernel": "levels"}).solve(want, b.to(dt))
+            s.solve(got, b.to(dt))
+            assert torch.equal(got, want)
+            want.zero_()
+            got.zero_()
+            gb.Solver(A, {"type": "PBiCGStab", "maxIterations": 4,
+                          "preconditioner": {"type": "ILU", "kernel": "levels"}}).solve(want, b.to(dt))
+            p.solve(got, b.to(dt))
+            assert torch.equal(got, want)
+    assert s.sweepKernel(F64) == "ring"
