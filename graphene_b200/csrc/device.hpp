@@ -415,8 +415,11 @@ HostDirect buildDirect(const HostMatrix& H, RingKind kind, bool dilu, i32 warps,
 // entries and their order, and the dependency order between barriers.
 // Throws GR_EINVAL.
 void checkDirect(const HostMatrix& H, const HostDirect& D);
+// Device copy of a plan. `accepted`: the direct kernels take the pattern;
+// `resident`: the tables are on the device.
 struct DirectPlan {
   RingKind kind = RingKind::Ilu;
+  bool accepted = false, resident = false;
   bool dilu = false, second = false, gsInPlace = false;
   bool longForward = false;  // ILU: the forward sweep has rows of more than three entries
   i32 warps = 1, maxSteps = 0;
@@ -505,8 +508,10 @@ struct DeviceMatrix {
                        RingKind kind = RingKind::Ilu, bool records = false);
 
   std::map<std::tuple<int, bool, i32>, std::unique_ptr<DirectPlan>> directPlans;  // [(kind, dilu, warps)]
-  // nullptr when the direct kernels cannot run this sweep.
-  DirectPlan* directPlan(RingKind kind, bool dilu, i32 warps);
+  // nullptr when the direct kernels cannot run this sweep, or a block that
+  // copies `depth` steps ahead over double vectors does not fit smemMax; the
+  // tables are then not kept on the device.
+  DirectPlan* directPlan(RingKind kind, bool dilu, i32 warps, i32 depth, size_t smemMax);
 
   // Device error word written by kernels whose bounded waits ran out
   // (GR_ETIMEOUT); 0 when clean.

@@ -527,14 +527,14 @@ DirectShape directShape(const HostMatrix& H, RingKind kind, DType coefficients, 
   return {warps, depth};
 }
 
-DirectPlan* DeviceMatrix::directPlan(RingKind kind, bool dilu, i32 warps) {
-  auto key = std::make_tuple(static_cast<int>(kind), dilu, warps);
-  auto it = directPlans.find(key);
-  if (it != directPlans.end()) return it->second.get();
-  std::unique_ptr<DirectPlan> R;
-  if (directFits(*host, kind)) {
+DirectPlan* DeviceMatrix::directPlan(RingKind kind, bool dilu, i32 warps, i32 depth, size_t smemMax) {
+  std::unique_ptr<DirectPlan>& slot = directPlans[std::make_tuple(static_cast<int>(kind), dilu, warps)];
+  auto usable = [&](const DirectPlan& R) { return R.accepted && directSmem(R, vt, DType::F64, depth) <= smemMax; };
+  if (slot && (slot->resident || !usable(*slot))) return usable(*slot) ? slot.get() : nullptr;
+  auto R = std::make_unique<DirectPlan>();
+  R->accepted = directFits(*host, kind);
+  if (R->accepted) {
     const HostDirect D = buildDirect(*host, kind, dilu, warps, vt);
-    R = std::make_unique<DirectPlan>();
     R->kind = kind;
     R->dilu = dilu;
     R->second = D.second;
@@ -546,31 +546,33 @@ DirectPlan* DeviceMatrix::directPlan(RingKind kind, bool dilu, i32 warps) {
     R->units = D.units;
     R->maxRows = D.maxRows;
     R->maxXSlots = D.maxXSlots;
-    R->src.upload(D.src);
-    R->tail.upload(D.tail);
-    if (D.second) {
-      R->src2.upload(D.src2);
-      R->tail2.upload(D.tail2);
-    }
-    R->factors = D.factors;
-    if (D.factors) {
-      R->levelStart.upload(D.levelStart);
-      R->levels.upload(D.levels);
-      R->transposed.upload(D.transposed);
-      if (D.longForward) R->transposed2.upload(D.transposed2);
-    }
-    R->steps.upload(D.steps);
-    R->stepStart.upload(D.stepStart);
-    R->stepRecord.upload(D.stepRecord);
-    R->stepUnit.upload(D.stepUnit);
-    if (kind != RingKind::Ilu) {
-      R->haloStart.upload(D.haloStart);
-      if (!D.haloSrc.empty()) R->haloSrc.upload(D.haloSrc);
+    if (usable(*R)) {
+      R->src.upload(D.src);
+      R->tail.upload(D.tail);
+      if (D.second) {
+        R->src2.upload(D.src2);
+        R->tail2.upload(D.tail2);
+      }
+      R->factors = D.factors;
+      if (D.factors) {
+        R->levelStart.upload(D.levelStart);
+        R->levels.upload(D.levels);
+        R->transposed.upload(D.transposed);
+        if (D.longForward) R->transposed2.upload(D.transposed2);
+      }
+      R->steps.upload(D.steps);
+      R->stepStart.upload(D.stepStart);
+      R->stepRecord.upload(D.stepRecord);
+      R->stepUnit.upload(D.stepUnit);
+      if (kind != RingKind::Ilu) {
+        R->haloStart.upload(D.haloStart);
+        if (!D.haloSrc.empty()) R->haloSrc.upload(D.haloSrc);
+      }
+      R->resident = true;
     }
   }
-  DirectPlan* out = R.get();
-  directPlans[key] = std::move(R);
-  return out;
+  slot = std::move(R);
+  return usable(*slot) ? slot.get() : nullptr;
 }
 
 }  // namespace gr

@@ -106,10 +106,10 @@ class IluNode : public Node {
       const DirectShape wide = directShapeFor(A, RingKind::Ilu, DType::F64);
       depth_ = own.depth;
       wideDepth_ = wide.warps > 0 ? wide.depth : own.depth;
-      DirectPlan* P = own.warps > 0 ? A.directPlan(RingKind::Ilu, dilu_, own.warps) : nullptr;
-      if (P && directSmem(*P, A.vt, DType::F64, std::max(depth_, wideDepth_)) <= smemMax) {
+      if (own.warps > 0)
+        direct_ = A.directPlan(RingKind::Ilu, dilu_, own.warps, std::max(depth_, wideDepth_), smemMax);
+      if (direct_) {
         kernel_ = 6;
-        direct_ = P;
         wideOther_ = wide.warps == 0;
       }
     }
@@ -312,14 +312,11 @@ class GsNode : public Node {
     // entries only for sweeps that start from x = 0.
     if (c.gsKernel == 0 && c.ringRecords && c.warpsPerBlock == 1 && !c.gsPairRows) {
       const i32 warps = directShapeFor(A, RingKind::GaussSeidel, A.vt).warps;
-      DirectPlan* P = warps > 0 ? A.directPlan(RingKind::GaussSeidel, false, warps) : nullptr;
-      DirectPlan* L = P ? A.directPlan(RingKind::GaussSeidelLower, false, warps) : nullptr;
       const size_t smemMax = static_cast<size_t>(maxDynamicSmem(A));
-      if (P && L && directSmem(*P, A.vt, DType::F64, kDirectGsDepth) <= smemMax &&
-          directSmem(*L, A.vt, DType::F64, kDirectGsDepth) <= smemMax) {
-        direct_ = P;
-        directLo_ = L;
-      }
+      auto plan = [&](RingKind kind) { return A.directPlan(kind, false, warps, kDirectGsDepth, smemMax); };
+      if (warps > 0) direct_ = plan(RingKind::GaussSeidel);
+      if (direct_) directLo_ = plan(RingKind::GaussSeidelLower);
+      if (!directLo_) direct_ = nullptr;
     }
     if (c.gsKernel != 2 && !direct_) {
       try {

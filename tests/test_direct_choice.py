@@ -104,3 +104,28 @@ def test_double_vectors_over_float_coefficients():
             p.solve(got, b.to(dt))
             assert torch.equal(got, want)
     assert s.sweepKernel(F64) == "ring"
+
+
+@pytest.mark.gpu
+def test_no_tables_for_a_sweep_that_does_not_fit():
+    """Tiles whose step tables outgrow shared memory: the matrix keeps no
+    direct tables (about 125 MB here) beside what the automatic choice makes
+    when an option of the ring kernel rules them out."""
+    import torch
+    from cuda.bindings import runtime
+    torch.cuda.init()
+    pool = runtime.cudaDeviceGetDefaultMemPool(0)[1]
+    h = gb.generate3DPoissonMatrix(F32, 256000, 1, 1, 16, gb.PART_CONTIGUOUS)
+
+    def held(cfg):
+        A = h.copyToTile()
+        before = int(runtime.cudaMemPoolGetAttribute(pool, runtime.cudaMemPoolAttr.cudaMemPoolAttrUsedMemCurrent)[1])
+        s = gb.Solver(A, cfg)
+        after = int(runtime.cudaMemPoolGetAttribute(pool, runtime.cudaMemPoolAttr.cudaMemPoolAttrUsedMemCurrent)[1])
+        return after - before, s.sweepKernel(F32), A, s
+
+    auto = held({"type": "ILU"})
+    assert not auto[1].startswith("direct")
+    same = held({"type": "ILU", "tilesPerBlock": 1})
+    assert same[1] == auto[1]
+    assert auto[0] - same[0] < 8 << 20
