@@ -12,6 +12,7 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <new>
 
 #include "config.hpp"
 #include "krylov.hpp"
@@ -75,6 +76,17 @@ DirectShape directShapeFor(const DeviceMatrix& A, RingKind kind, DType vec) {
   return directShape(*A.host, kind, A.vt, vec, A.numSMs, perSM);
 }
 
+// nullptr also when the tables exceed their limits or memory: the other
+// kernels need less.
+DirectPlan* directPlanOrNull(DeviceMatrix& A, RingKind kind, bool dilu, i32 warps, i32 depth, size_t smemMax) {
+  try {
+    return A.directPlan(kind, dilu, warps, depth, smemMax);
+  } catch (const Error&) {
+  } catch (const std::bad_alloc&) {
+  }
+  return nullptr;
+}
+
 std::string directName(const DirectPlan& P, i32 depth) {
   return "direct " + std::to_string(P.warps) + "x" + std::to_string(depth);
 }
@@ -107,7 +119,7 @@ class IluNode : public Node {
       depth_ = own.depth;
       wideDepth_ = wide.warps > 0 ? wide.depth : own.depth;
       if (own.warps > 0)
-        direct_ = A.directPlan(RingKind::Ilu, dilu_, own.warps, std::max(depth_, wideDepth_), smemMax);
+        direct_ = directPlanOrNull(A, RingKind::Ilu, dilu_, own.warps, std::max(depth_, wideDepth_), smemMax);
       if (direct_) {
         kernel_ = 6;
         wideOther_ = wide.warps == 0;
@@ -169,6 +181,7 @@ class IluNode : public Node {
     try {
       wide_ = std::make_unique<IluNode>(A_, cfg_, false);
     } catch (const Error&) {  // no room for it: the direct kernel serves both types
+    } catch (const std::bad_alloc&) {
     }
     if (wide_ && wide_->kernel_ != 4) wide_.reset();  // likewise without the ring
   }
@@ -313,7 +326,7 @@ class GsNode : public Node {
     if (c.gsKernel == 0 && c.ringRecords && c.warpsPerBlock == 1 && !c.gsPairRows) {
       const i32 warps = directShapeFor(A, RingKind::GaussSeidel, A.vt).warps;
       const size_t smemMax = static_cast<size_t>(maxDynamicSmem(A));
-      auto plan = [&](RingKind kind) { return A.directPlan(kind, false, warps, kDirectGsDepth, smemMax); };
+      auto plan = [&](RingKind kind) { return directPlanOrNull(A, kind, false, warps, kDirectGsDepth, smemMax); };
       if (warps > 0) direct_ = plan(RingKind::GaussSeidel);
       if (direct_) directLo_ = plan(RingKind::GaussSeidelLower);
       if (!directLo_) direct_ = nullptr;
