@@ -496,6 +496,7 @@ void HostMatrix::buildLevels() {
   upperLevel.assign(n, 0);
   nLowerLevels.assign(P, 0);
   nUpperLevels.assign(P, 0);
+  std::vector<i64> lower8(P, 0), upper8(P, 0);
   parallelFor(P, [&](i64 T) {
     const i64 base = tileStart[T];
     const i64 nRows = tiles[T].rows();
@@ -525,7 +526,21 @@ void HostMatrix::buildLevels() {
     }
     nLowerLevels[T] = maxL + 1;
     nUpperLevels[T] = maxU + 1;
+    auto rounded = [&](const std::vector<i32>& level, i32 levels) {
+      std::vector<i64> size(levels, 0);
+      for (i64 p = base; p < base + nRows; ++p) ++size[level[p]];
+      i64 sum = 0;
+      for (i64 k : size) sum += (k + 7) / 8 * 8;
+      return sum;
+    };
+    lower8[T] = rounded(lowerLevel, maxL + 1);
+    upper8[T] = rounded(upperLevel, maxU + 1);
   });
+  lowerRows8 = upperRows8 = 0;
+  for (i32 T = 0; T < P; ++T) {
+    lowerRows8 += lower8[T];
+    upperRows8 += upper8[T];
+  }
   // "Multicolour recommended" when more than 90 % of the rows sit in colours
   // holding more than 12 rows (CRSHostMatrix.cpp:648-669).
   i64 parallelRows = 0;

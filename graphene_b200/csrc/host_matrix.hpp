@@ -73,6 +73,9 @@ struct HostMatrix {
   // Level ("colour") of each row in its tile's lower / upper dependency DAG.
   std::vector<i32> lowerLevel, upperLevel;  // tile order
   std::vector<i32> nLowerLevels, nUpperLevels;  // per tile
+  // Rows of the lower / upper levels, each level rounded up to 8 rows (what
+  // the direct sweeps store).
+  i64 lowerRows8 = 0, upperRows8 = 0;
   bool multicolorRecommended = false;
 
   i64 numHaloTotal = 0;

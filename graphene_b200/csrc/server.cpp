@@ -24,12 +24,27 @@ i64 estimateFootprint(const HostMatrix& H, const std::string& json, DType t) {
   const i64 rows = n * (vs + 8) + 4 * (H.P + 1);                 // diagonal, tile starts, permutation
   const i64 localCrs = 4 * (n + 1) + m * (4 + vs);
   const i64 stream = 2 * (m * (4 + vs) + n * (8 + 2 * vs) + 64 * (i64(H.P) + 1));  // template + packed copy
-  // The direct sweeps' sources and packed records: at most 3 x 64 bytes a row
-  // and sweep, padding included.
-  const i64 direct = 2 * 192 * n;
+  // The direct sweeps' tables and packed records, as if every row had a second
+  // triple: 40 bytes of sources a record and its packed form (float: two
+  // triples, tail and third slot; double: the same in 16-byte words), 12 bytes
+  // a step word; ILU adds 32 bytes of transposes a forward record and 16 a
+  // level. Gauss-Seidel keeps two such sweeps over the lower levels.
+  const i64 record = 40 + (vs == 4 ? 44 : 72);
+  i64 lowerLevels = 0, upperLevels = 0;
+  for (i32 T = 0; T < H.P; ++T) {
+    lowerLevels += H.nLowerLevels[T];
+    upperLevels += H.nUpperLevels[T];
+  }
+  const i64 words = 12 * (n / 32 + 32 * i64(H.P));  // full steps, table ends
+  const i64 iluDirect = record * (H.lowerRows8 + H.upperRows8) + 32 * H.lowerRows8 + 28 * lowerLevels +
+                        12 * upperLevels + 2 * words;
+  const i64 gsDirect = 2 * (record * H.lowerRows8 + 12 * lowerLevels + words) + 4 * H.numHaloTotal;
+  const i64 direct = std::max(iluDirect, gsDirect);
+  // Double vectors over float coefficients may keep a ring beside them.
+  const i64 sweeps = vs == 4 && t == DType::F64 ? stream + direct : std::max(stream, direct);
   const i64 factors = m * vs + n * vs;
   const i64 vectors = 16 * n * std::max<i64>(8, static_cast<i64>(dtypeSize(t)));     // Krylov, MPIR, staging
-  return sell + rows + localCrs + std::max(stream, direct) + factors + vectors + (i64(4) << 20);
+  return sell + rows + localCrs + sweeps + factors + vectors + (i64(4) << 20);
 }
 
 struct Server::Entry {

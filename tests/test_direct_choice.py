@@ -2,8 +2,9 @@
 (directShape, direct.cpp): the shape it gives for matrices on each side of its
 lines, and what solvers then run."""
 import ctypes as C
+import subprocess
+import sys
 
-import numpy as np
 import pytest
 
 import graphene_b200 as gb
@@ -129,3 +130,42 @@ def test_no_tables_for_a_sweep_that_does_not_fit():
     same = held({"type": "ILU", "tilesPerBlock": 1})
     assert same[1] == auto[1]
     assert auto[0] - same[0] < 8 << 20
+
+
+FOOTPRINT = """
+import sys
+import numpy as np
+import torch
+from cuda.bindings import runtime
+import graphene_b200 as gb
+torch.cuda.init()
+pool = runtime.cudaDeviceGetDefaultMemPool(0)[1]
+def held():
+    return int(runtime.cudaMemPoolGetAttribute(pool, runtime.cudaMemPoolAttr.cudaMemPoolAttrUsedMemCurrent)[1])
+nx, ny, tiles, t = map(int, sys.argv[1:5])
+h = gb.generate3DPoissonMatrix(t, nx, ny, 1, tiles, gb.PART_CONTIGUOUS)
+cfg = {"type": "PBiCGStab", "maxIterations": 2, "preconditioner": {"type": "ILU"}}
+dt = np.float64 if t or len(sys.argv) > 5 else np.float32
+before = held()
+A = h.copyToTile()
+s = gb.Solver(A, cfg)
+s.solveHost(np.zeros(h.numRows, dt), np.ones(h.numRows, dt))
+used = held() - before
+assert s.sweepKernel(t).startswith("direct")
+srv = gb.Server(slots=1)
+print(used, srv.wait(srv.submit(h, cfg, np.ones(h.numRows, dt)))[2]["footprint_bytes"])
+srv.close()
+"""
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("args", [("65536", "1", "64", "0"), ("65536", "1", "64", "1"), ("20000", "3", "100", "0"),
+                                  ("20000", "3", "100", "0", "double"), ("300", "300", "60", "1")])
+def test_server_admits_by_no_less_than_a_pair_holds(args):
+    """Narrow levels, each padded to eight records: what the matrix and its
+    solver hold (in a process of its own, with no blocks kept from before)
+    stays within the estimate that the server admits by."""
+    out = subprocess.run([sys.executable, "-c", FOOTPRINT, *args], capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0, out.stderr
+    used, estimate = map(int, out.stdout.split())
+    assert 0 < used <= estimate
