@@ -437,6 +437,7 @@ size_t directSmem(const DirectPlan& P, DType coefficients, DType W, i32 depth);
 struct DirectShape {
   i32 warps = 0, depth = 0;
 };
+double rowsPerLevel(const HostMatrix& H);  // of the forward sweeps
 constexpr i32 kDirectGsDepth = 4;  // Gauss-Seidel sweeps are built for this depth only
 // The choice for vectors of type `vec` on a device with numSMs SMs of
 // smemPerSM bytes of shared memory (rule and figures: direct.cpp).

@@ -426,6 +426,12 @@ size_t directSmem(const DirectPlan& P, DType coefficients, DType W, i32 depth) {
          static_cast<size_t>((P.maxXSlots + 3) / 4 * 4 + rhs) * dtypeSize(W) + 4 * static_cast<size_t>(P.maxSteps);
 }
 
+double rowsPerLevel(const HostMatrix& H) {
+  i64 levels = 1;
+  for (i32 l : H.nLowerLevels) levels += l;
+  return static_cast<double>(H.n) / static_cast<double>(levels);
+}
+
 // What counts is how many tiles share an SM (t), how many rows a level has,
 // how many tiles are resident at once, and whether the sweep's data stay in
 // L2; results do not depend on the shape. All figures: us on B200, level ring
@@ -478,12 +484,9 @@ size_t directSmem(const DirectPlan& P, DType coefficients, DType W, i32 depth) {
 DirectShape directShape(const HostMatrix& H, RingKind kind, DType coefficients, DType vec, i32 numSMs,
                         i64 smemPerSM) {
   const bool gs = kind != RingKind::Ilu, f32 = coefficients == DType::F32;
-  i64 levels = 1, halo = 0;
-  for (i32 T = 0; T < H.P; ++T) {
-    levels += H.nLowerLevels[T];
-    halo = std::max(halo, H.tiles[T].nHalo);
-  }
-  const double t = static_cast<double>(H.P) / numSMs, rows = static_cast<double>(H.n) / static_cast<double>(levels);
+  i64 halo = 0;
+  for (const HostMatrix::Tile& tile : H.tiles) halo = std::max(halo, tile.nHalo);
+  const double t = static_cast<double>(H.P) / numSMs, rows = rowsPerLevel(H);
   // Waves of blocks with room for second triples, copying d steps ahead.
   const i64 vs = static_cast<i64>(dtypeSize(vec)), rec = f32 ? 44 : 72;
   auto waves = [&](i32 warps, i32 d) {

@@ -581,8 +581,14 @@ __global__ void __launch_bounds__(32 * WARPS) gsDirectKernel(DirectView V, SPro<
 }
 
 // A solver's blocks from a plan's sources, the factor (or matrix) values F in
-// tile-local CRS order and the diagonal inv in tile order. One thread block
-// per tile, a warp per step; a record's row gives its diagonal.
+// tile-local CRS order and the diagonal inv in tile order; a record's row
+// gives its diagonal. gridDim.y blocks a tile; a warp a step, or eight lanes
+// (whose 16-byte words fill a line) where steps have less than 16 rows: a
+// step is a chain of three loads, so what counts is steps in flight. Both
+// plans of a Gauss-Seidel solver, with its wait, with one block a tile and a
+// warp a step -> now: a chain of 4096 rows a tile, 16 tiles, 1018 us -> 35; a
+// 96^3 grid in 148 tiles 147 us -> 57. An eight-lane step of 128 rows is
+// slower than a warp's (16^3 in one tile: 48 us, 30).
 template <class MV>
 __global__ void __launch_bounds__(256) directPackKernel(const int* __restrict__ tileStart,
                                                         const int* __restrict__ stepStart,
@@ -592,8 +598,9 @@ __global__ void __launch_bounds__(256) directPackKernel(const int* __restrict__ 
                                                         const int4* __restrict__ src, const int4* __restrict__ src2,
                                                         const uint32_t* __restrict__ tail,
                                                         const uint32_t* __restrict__ tail2, const MV* __restrict__ F,
-                                                        const MV* __restrict__ inv, uint4* __restrict__ data) {
-  const int base = tileStart[blockIdx.x], lane = threadIdx.x & 31;
+                                                        const MV* __restrict__ inv, uint4* __restrict__ data,
+                                                        int lanesLog2) {
+  const int base = tileStart[blockIdx.x], lanes = 1 << lanesLog2, lane = threadIdx.x & (lanes - 1);
   auto val = [&](int e) { return e >= 0 ? F[e] : MV(0); };
   auto put = [&](char* out, uint32_t plane, const int4 s, uint32_t last) {
     if constexpr (sizeof(MV) == 4) {
@@ -607,12 +614,12 @@ __global__ void __launch_bounds__(256) directPackKernel(const int* __restrict__ 
           make_uint4(__double2loint(v2), __double2hiint(v2), static_cast<uint32_t>(s.w), last);
     }
   };
-  for (int i = stepStart[blockIdx.x] + kDirectHead + static_cast<int>(threadIdx.x >> 5);
-       i < stepStart[blockIdx.x + 1]; i += static_cast<int>(blockDim.x >> 5)) {
+  for (int i = stepStart[blockIdx.x] + kDirectHead + static_cast<int>((blockIdx.y * blockDim.x + threadIdx.x) >> lanesLog2);
+       i < stepStart[blockIdx.x + 1]; i += static_cast<int>((gridDim.y * blockDim.x) >> lanesLog2)) {
     const uint32_t w = steps[i], rows = w & 0xFFu, nLong = (w >> kDirectLongShift) & 0xFFu;
     const DirectBlock<sizeof(MV)> at(w, (w & kDirectDiag) != 0);
     char* blk = reinterpret_cast<char*>(data + stepUnit[i]);
-    for (uint32_t q = lane; q < rows; q += 32) {
+    for (uint32_t q = lane; q < rows; q += lanes) {
       const size_t p = stepRecord[i] + q;
       const uint32_t t = tail[p];
       put(blk + 16 * q, at.plane, src[p], t);
@@ -835,12 +842,16 @@ size_t directBytes(const DirectPlan& P) { return 16 * std::max<size_t>(1, static
 
 void launchDirectPack(DeviceMatrix& A, const DirectPlan& P, DBuf& data, const void* F, const void* inv,
                       cudaStream_t s) {
+  const int perTile = std::clamp(8 * A.numSMs / std::max<int>(1, A.P), 1, 32);
+  const i64 sweeps = P.kind == RingKind::Ilu ? 2 : 1;
+  const int lanesLog2 = sweeps * P.maxRows >= 16 * P.maxSteps ? 5 : 3;
   auto go = [&](auto zero) {
     using MV = decltype(zero);
-    dev::directPackKernel<MV><<<A.P, 256, 0, s>>>(
+    dev::directPackKernel<MV><<<dim3(A.P, perTile), 256, 0, s>>>(
         A.tileStart.as<int>(), P.stepStart.as<int>(), P.steps.as<uint32_t>(), P.stepRecord.as<uint32_t>(),
         P.stepUnit.as<uint32_t>(), P.src.as<int4>(), P.second ? P.src2.as<int4>() : nullptr, P.tail.as<uint32_t>(),
-        P.second ? P.tail2.as<uint32_t>() : nullptr, static_cast<const MV*>(F), static_cast<const MV*>(inv), data.as<uint4>());
+        P.second ? P.tail2.as<uint32_t>() : nullptr, static_cast<const MV*>(F), static_cast<const MV*>(inv), data.as<uint4>(),
+        lanesLog2);
   };
   if (A.vt == DType::F32) go(0.0f);
   else go(0.0);

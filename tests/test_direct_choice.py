@@ -169,3 +169,46 @@ def test_server_admits_by_no_less_than_a_pair_holds(args):
     assert out.returncode == 0, out.stderr
     used, estimate = map(int, out.stdout.split())
     assert 0 < used <= estimate
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [F32, F64])
+@pytest.mark.parametrize("dims,tiles,factor", [((3000, 1, 1), 2, True), ((6000, 1, 1), 300, False),
+                                               ((16, 16, 16), 1, True), ((40, 38, 3), 7, True)])
+def test_packing_of_narrow_and_wide_steps(dims, tiles, factor, dtype):
+    """Several blocks a tile, eight lanes or a warp a step, chains with and
+    without the fused factorisation: as the level schedules, bit for bit, also
+    after new values."""
+    import torch
+    h = gb.generate3DPoissonMatrix(dtype, *dims, tiles, gb.PART_CONTIGUOUS)
+    A = h.copyToTile()
+    dt = torch.float64 if dtype == F64 else torch.float32
+    b = torch.linspace(-1, 1, h.numRows, dtype=dt, device="cuda")
+    rp, col, off, dg = h.globalCrs()
+    ilu, gs = {"type": "ILU"}, {"type": "GaussSeidel", "numFixedIterations": 2}
+    solvers = [gb.Solver(A, c) for c in (ilu, gs)]
+    assert solvers[0].sweepKernel(dtype).endswith("factor") == factor
+    for scale in (1.0, 1.5):
+        A.updateGlobalValues(off * scale, dg * 2)
+        for c, s in zip((ilu, gs), solvers):
+            s.refresh()
+            got, want = torch.ones_like(b), torch.ones_like(b)
+            s.solve(got, b)
+            gb.Solver(A, {**c, "kernel": "levels"}).solve(want, b)
+            assert torch.equal(got, want)
+
+
+@pytest.mark.gpu
+def test_refresh_of_long_chains():
+    """New values in a Gauss-Seidel solver of few tiles and many narrow levels
+    take tens of microseconds (a block a tile took a millisecond)."""
+    import time
+    h = gb.generate3DPoissonMatrix(F32, 65536, 1, 1, 16, gb.PART_CONTIGUOUS)
+    s = gb.Solver(h.copyToTile(), {"type": "GaussSeidel", "numFixedIterations": 1})
+    assert s.sweepKernel() == "direct 4x4"
+    best = 1.0
+    for _ in range(10):
+        t0 = time.perf_counter()
+        s.refresh()
+        best = min(best, time.perf_counter() - t0)
+    assert best < 3e-4
