@@ -46,8 +46,8 @@ class DBuf {
   void* get() const { return p_; }
   template <class T> T* as() const { return static_cast<T*>(p_); }
   size_t bytes() const { return bytes_; }
-  template <class T>
-  void upload(const std::vector<T>& v) {
+  template <class T, class Alloc>
+  void upload(const std::vector<T, Alloc>& v) {
     alloc(std::max<size_t>(1, v.size()) * sizeof(T));
     if (!v.empty()) GR_CUDA(cudaMemcpy(p_, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
   }
@@ -380,6 +380,25 @@ struct DirectBlock {
     return (rows + kDirectAlign - 1) & ~(kDirectAlign - 1);
   }
 };
+// A vector that resize() leaves uninitialised: the tables' pages are first
+// touched by the threads that fill them.
+template <class T>
+struct RawAllocator : std::allocator<T> {
+  template <class U>
+  struct rebind {
+    using other = RawAllocator<U>;
+  };
+  template <class U>
+  void construct(U* p) noexcept {
+    ::new (static_cast<void*>(p)) U;
+  }
+  template <class U, class... Args>
+  void construct(U* p, Args&&... args) {
+    ::new (static_cast<void*>(p)) U(std::forward<Args>(args)...);
+  }
+};
+template <class T>
+using RawVector = std::vector<T, RawAllocator<T>>;
 struct HostDirect {
   RingKind kind = RingKind::Ilu;
   bool dilu = false, second = false, gsInPlace = false;  // second: some row has more than three entries
@@ -391,13 +410,13 @@ struct HostDirect {
   // triple's values (-1: padding) and its first two slots (4 c0 | 4 c1 <<
   // 16); the third slot and the row (4 slot | 4 row << 16) in tail. second:
   // the second triple's in src2 and its third slot in tail2.
-  std::vector<int4> src, src2;
-  std::vector<uint32_t> tail, tail2;
-  std::vector<uint32_t> steps;
+  RawVector<int4> src, src2;
+  RawVector<uint32_t> tail, tail2;
+  RawVector<uint32_t> steps;
   std::vector<i32> stepStart;  // P + 1
   // Per step word: the step's first record and the first 16-byte unit of its
   // block.
-  std::vector<uint32_t> stepRecord, stepUnit;
+  RawVector<uint32_t> stepRecord, stepUnit;
   std::vector<i32> haloStart, haloSrc;
   // The factorisation in the forward sweep's order (ILU, when `factors`): per
   // level {first record, rows | long rows << 16, first step word, first
@@ -405,7 +424,7 @@ struct HostDirect {
   // CRS entries (column, row) of its entries (-1: none).
   bool factors = false;
   std::vector<i32> levelStart;
-  std::vector<int4> levels, transposed, transposed2;
+  RawVector<int4> levels, transposed, transposed2;
 };
 // Whether the direct kernels can run a sweep of H (every row of the sweep
 // has at most 6 entries and a tile's slots fit 16 bits).

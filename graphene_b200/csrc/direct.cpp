@@ -116,11 +116,13 @@ HostDirect buildDirect(const HostMatrix& H, RingKind kind, bool dilu, i32 warps,
   std::vector<std::vector<uint32_t>> tileSteps(H.P);
   std::vector<std::vector<i32>> order(H.P);  // record -> tile-local row, -1: padding
   std::vector<i64> nForward(H.P, 0);         // records of the forward sweep
+  std::vector<i64> tileUnits(H.P, 0);        // 16-byte units of a tile's blocks
   std::atomic<bool> second{false}, longForward{false};
   parallelFor(H.P, [&](i64 T) {
     const i64 base = H.tileStart[T], nRows = H.tileStart[T + 1] - base;
     std::vector<uint32_t>& st = tileSteps[T];
     std::vector<i32>& ord = order[T];
+    bool tileSecond = false, tileLongForward = false;
     st.assign(kDirectHead, 0u);
     for (int sweep = 0; sweep < (gs ? 1 : 2); ++sweep) {
       const bool upper = sweep == 1;
@@ -134,8 +136,8 @@ HostDirect buildDirect(const HostMatrix& H, RingKind kind, bool dilu, i32 warps,
         int c = 0;
         eachEntry(H, kind, upper, base + r, r, nRows, [&](i64) { ++c; });
         if (c > 3) {
-          second = true;
-          if (!upper) longForward = true;
+          tileSecond = true;
+          if (!upper) tileLongForward = true;
           isLong[r] = 1;
           ++longs[l];
         }
@@ -161,7 +163,10 @@ HostDirect buildDirect(const HostMatrix& H, RingKind kind, bool dilu, i32 warps,
           if (i64& q = next[lev[base + r]]; q >= 0 && isLong[r] == want) ord[q++] = static_cast<i32>(r);
       if (!upper) nForward[T] = size;
     }
+    for (size_t i = kDirectHead; i < st.size(); ++i) tileUnits[T] += blockBytes(D.valueBytes, st[i]) / 16;
     st.resize(st.size() + kDirectAhead, 0u);
+    if (tileSecond) second = true;
+    if (tileLongForward) longForward = true;
   });
   D.second = second;
   D.longForward = longForward;
@@ -174,39 +179,48 @@ HostDirect buildDirect(const HostMatrix& H, RingKind kind, bool dilu, i32 warps,
     D.maxRows = std::max<i64>(D.maxRows, H.tileStart[T + 1] - H.tileStart[T]);
     D.maxXSlots = std::max(D.maxXSlots, xSlotsOf(H, kind, D.gsInPlace, T));
   }
+  std::vector<i64> unitStart(H.P + 1, 0);
+  for (i32 T = 0; T < H.P; ++T) unitStart[T + 1] = unitStart[T] + tileUnits[T];
   D.records = recStart[H.P];
-  D.steps.reserve(D.stepStart[H.P]);
-  D.stepRecord.reserve(D.stepStart[H.P]);
-  D.stepUnit.reserve(D.stepStart[H.P]);
-  i64 rec = 0;
-  for (const auto& st : tileSteps)
-    for (size_t i = 0; i < st.size(); ++i) {
-      const uint32_t w = st[i];
-      const bool step = i >= static_cast<size_t>(kDirectHead);
-      const i64 rows = step ? (static_cast<i64>(w & 0xFFu) + kDirectAlign - 1) / kDirectAlign * kDirectAlign : 0;
-      const i64 units = step ? blockBytes(D.valueBytes, w) / 16 : 0;
-      D.steps.push_back(step ? w | static_cast<uint32_t>(units) << kDirectUnitShift : w);
-      D.stepRecord.push_back(static_cast<uint32_t>(rec));
-      D.stepUnit.push_back(static_cast<uint32_t>(D.units));
-      rec += rows;
-      D.units += units;
-    }
+  D.units = unitStart[H.P];
   if (D.records >= (i64(1) << 31) || D.units >= (i64(1) << 32))
     fail(GR_EUNSUPPORTED, "direct sweep exceeds 2^31 records");
+  D.steps.resize(D.stepStart[H.P]);
+  D.stepRecord.resize(D.stepStart[H.P]);
+  D.stepUnit.resize(D.stepStart[H.P]);
   const int4 none = make_int4(-1, -1, -1, 0);
-  D.src.assign(D.records, none);
-  D.tail.assign(D.records, 0u);
+  D.src.resize(D.records);
+  D.tail.resize(D.records);
   if (D.second) {
-    D.src2.assign(D.records, none);
-    D.tail2.assign(D.records, 0u);
+    D.src2.resize(D.records);
+    D.tail2.resize(D.records);
   }
   parallelFor(H.P, [&](i64 T) {
     const i64 base = H.tileStart[T], nRows = H.tileStart[T + 1] - base;
     const i64 start = gs && !D.gsInPlace ? nRows : 0;  // where sweep-start values live
     const uint32_t zero = static_cast<uint32_t>(4 * (xSlotsOf(H, kind, D.gsInPlace, T) - 1));
+    i64 at = D.stepStart[T], firstRecord = recStart[T], firstUnit = unitStart[T];
+    for (size_t i = 0; i < tileSteps[T].size(); ++i, ++at) {
+      const uint32_t w = tileSteps[T][i];
+      const bool step = i >= static_cast<size_t>(kDirectHead);
+      const i64 units = step ? blockBytes(D.valueBytes, w) / 16 : 0;
+      D.steps[at] = step ? w | static_cast<uint32_t>(units) << kDirectUnitShift : w;
+      D.stepRecord[at] = static_cast<uint32_t>(firstRecord);
+      D.stepUnit[at] = static_cast<uint32_t>(firstUnit);
+      if (step) firstRecord += (static_cast<i64>(w & 0xFFu) + kDirectAlign - 1) / kDirectAlign * kDirectAlign;
+      firstUnit += units;
+    }
     for (i64 q = 0; q < static_cast<i64>(order[T].size()); ++q) {
       const i64 r = order[T][q], rec = recStart[T] + q;
-      if (r < 0) continue;
+      if (r < 0) {
+        D.src[rec] = none;
+        D.tail[rec] = 0;
+        if (D.second) {
+          D.src2[rec] = none;
+          D.tail2[rec] = 0;
+        }
+        continue;
+      }
       i32 e[6] = {-1, -1, -1, -1, -1, -1};
       uint32_t c[6] = {zero, zero, zero, zero, zero, zero};
       int m = 0;
@@ -230,6 +244,14 @@ HostDirect buildDirect(const HostMatrix& H, RingKind kind, bool dilu, i32 warps,
     std::vector<i64> forward(H.P + 1, 0);  // forward records before each tile
     for (i32 T = 0; T < H.P; ++T) {
       forward[T + 1] = forward[T] + nForward[T];
+      D.levelStart[T + 1] = D.levelStart[T] + H.nLowerLevels[T] - (dilu || H.nLowerLevels[T] == 0 ? 0 : 1);
+    }
+    D.levels.resize(D.levelStart[H.P]);
+    D.transposed.resize(forward[H.P]);
+    if (D.longForward) D.transposed2.resize(forward[H.P]);
+    parallelFor(H.P, [&](i64 T) {
+      const i64 base = H.tileStart[T], nRows = H.tileStart[T + 1] - base;
+      i64 l = D.levelStart[T];
       int4 level = make_int4(-1, 0, 0, 0);
       for (uint32_t i = 0; i < D.steps[D.stepStart[T] + 1]; ++i) {
         const i64 at = D.stepStart[T] + kDirectHead + i;
@@ -240,19 +262,17 @@ HostDirect buildDirect(const HostMatrix& H, RingKind kind, bool dilu, i32 warps,
                             static_cast<int>(forward[T] + D.stepRecord[at] - recStart[T]));
         level.y += static_cast<int>((w & 0xFFu) | ((w >> kDirectLongShift) & 0xFFu) << 16);
         if (w & kDirectEnd) {
-          D.levels.push_back(level);
+          D.levels[l++] = level;
           level.x = -1;
         }
       }
-      D.levelStart[T + 1] = static_cast<i32>(D.levels.size());
-    }
-    D.transposed.assign(forward[H.P], none);
-    if (D.longForward) D.transposed2.assign(forward[H.P], none);
-    parallelFor(H.P, [&](i64 T) {
-      const i64 base = H.tileStart[T], nRows = H.tileStart[T + 1] - base;
       for (i64 q = 0; q < nForward[T]; ++q) {
         const i64 r = order[T][q];
-        if (r < 0) continue;
+        if (r < 0) {
+          D.transposed[forward[T] + q] = none;
+          if (D.longForward) D.transposed2[forward[T] + q] = none;
+          continue;
+        }
         i32 t[6] = {-1, -1, -1, -1, -1, -1};
         int m = 0;
         eachEntry(H, kind, false, base + r, r, nRows, [&](i64 k) { t[m++] = entryAt(H, base + H.colLocal[k], r); });
