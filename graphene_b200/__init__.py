@@ -694,6 +694,12 @@ class Batch:
         check(_lib.lib().gr_batch_solve_host(self._b, xa, ba, t, st))
         return xs, [SolverStats._from(s) for s in st]
 
+    def sweepKernel(self, t: int = FLOAT32) -> str:
+        """The kernel of the preconditioner's sweeps over vectors of type t (gr_batch_sweep_kernel)."""
+        buf = C.create_string_buffer(256)
+        check(_lib.lib().gr_batch_sweep_kernel(self._b, t, buf, 256))
+        return buf.value.decode()
+
     def close(self):
         b = getattr(self, "_b", None)
         if b and _lib is not None:

@@ -23,12 +23,14 @@ std::shared_ptr<HostMatrix> concatForBatch(const std::vector<std::shared_ptr<Hos
 
 class BatchSolve {
  public:
-  // json: a PBiCGStab configuration with the ILU preconditioner (run by the
-  // ring substitution kernel, one tile per block).
+  // json: a PBiCGStab configuration, or IterativeRefinement over one, whose
+  // preconditioner runs a block per tile: ILU (automatic or ring kernel) or
+  // Gauss-Seidel with a fixed number of iterations (automatic or block ring).
   BatchSolve(std::vector<std::shared_ptr<HostMatrix>> parts, const std::string& json);
   ~BatchSolve();
   // Host vectors in each system's natural order; x in/out.
   std::vector<gr_stats> solveHost(const std::vector<void*>& x, const std::vector<const void*>& b, DType t);
+  std::string sweepKernel(DType W) const { return tree_->sweepKernel(W); }
   int systems() const { return static_cast<int>(parts_.size()); }
 
  private:

@@ -850,6 +850,17 @@ int gr_batch_solve_host(gr_batch* b, void* const* x, const void* const* rhs, gr_
   });
 }
 
+int gr_batch_sweep_kernel(const gr_batch* b, gr_dtype vectors, char* buf, size_t len) {
+  return guarded([&] {
+    need(b, "batch");
+    need(buf, "buf");
+    if (len == 0) gr::fail(GR_EINVAL, "buffer length is 0");
+    const std::string k = b->b->sweepKernel(gr::toDType(vectors));
+    std::strncpy(buf, k.c_str(), len - 1);
+    buf[len - 1] = '\0';
+  });
+}
+
 void gr_batch_destroy(gr_batch* b) { delete b; }
 
 int gr_selftest_wait_timeout(int32_t* status, int64_t* elapsed_ns) {

@@ -586,14 +586,15 @@ class PbicgstabNode : public Node {
       gs_ = dynamic_cast<GsNode*>(pre_.get());
     }
     if (A.batch) {
-      // A batch keeps one state per system; its preconditioner must look
-      // up a block's system, which the block ring kernels (ILU substitution,
-      // Gauss-Seidel sweeps) do.
+      // A batch keeps one state per system; its preconditioner must look up a
+      // block's system, which the kernels with a block per tile do (direct
+      // sweeps, block rings).
       const bool iluOk = ilu_ && ilu_->batchKernel();
       const bool gsOk = gs_ && gs_->fusedPrologue() && gs_->blockPerTile();
       if (!iluOk && !gsOk)
-        fail(GR_EUNSUPPORTED, "batched PBiCGStab needs the ILU preconditioner with the ring kernel, or Gauss-Seidel "
-                              "with numFixedIterations > 0 on the block ring kernel");
+        fail(GR_EUNSUPPORTED, "batched PBiCGStab needs the ILU preconditioner with the automatic or ring kernel, or "
+                              "Gauss-Seidel with numFixedIterations > 0 on the automatic or block ring kernel, and "
+                              "tiles that fit shared memory");
       systems_ = A.batch->systems;
       GR_CUDA(cudaMallocHost(&host_, sizeof(KState) * systems_ + sizeof(int)));
       batchHost_ = true;

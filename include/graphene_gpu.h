@@ -578,14 +578,17 @@ void gr_server_destroy(gr_server* s);
  * own Krylov state and convergence test on the device, and a system that
  * has converged drops out of the work while the others continue. Each
  * system's result equals the result of solving it alone with the same
- * configuration. json: a PBiCGStab configuration with the ILU
- * preconditioner (the ring substitution kernel, one tile per block); the
- * systems share one coefficient type. */
+ * configuration. json: a PBiCGStab configuration, or IterativeRefinement
+ * over one, with the ILU preconditioner (automatic or ring kernel) or
+ * Gauss-Seidel with a fixed number of iterations (automatic or block ring
+ * kernel); the systems share one coefficient type. */
 typedef struct gr_batch gr_batch;
 int gr_batch_create(gr_host_matrix* const* systems, int32_t count, const char* json, gr_batch** out);
 /* x[i] (in: initial guess, out: solution) and b[i]: host vectors of system i
  * in natural order, type t; stats: count entries (may be NULL). */
 int gr_batch_solve_host(gr_batch* b, void* const* x, const void* const* rhs, gr_dtype t, gr_stats* stats);
+/* gr_solver_sweep_kernel for the batch's preconditioner. */
+int gr_batch_sweep_kernel(const gr_batch* b, gr_dtype vectors, char* buf, size_t len);
 void gr_batch_destroy(gr_batch* b);
 
 /* ---- self-test ----------------------------------------------------------

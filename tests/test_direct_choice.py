@@ -212,3 +212,37 @@ def test_refresh_of_long_chains():
         s.refresh()
         best = min(best, time.perf_counter() - t0)
     assert best < 3e-4
+
+
+# Every shape the ILU rule can give, each at its smallest matrix or nearly so.
+SHAPES = {
+    "direct 2x8": (lambda: grid(24, 27), F32),
+    "direct 4x8": (lambda: grid(32, 8), F32),
+    "direct 1x8": (lambda: gb.generate3DPoissonMatrix(F32, 29, 28, 27, 330, gb.PART_RCB), F32),
+    "direct 1x4": (lambda: gb.generate3DPoissonMatrix(F32, 36, 35, 34, 2900, gb.PART_RCB), F32),
+    "direct 2x4": (lambda: mesh(100, 800), F64),
+    "direct 4x4": (lambda: grid(96, 160), F64),
+}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", sorted(SHAPES))
+def test_every_ilu_shape(name):
+    """Taken, and as the level schedules, in either type of vectors."""
+    import torch
+    make, coef = SHAPES[name]
+    h = make() if coef == F32 else make().astype(coef)
+    A = h.copyToTile()
+    n = h.numRows
+    g = torch.Generator().manual_seed(9)
+    b64 = torch.rand(n + 1, generator=g, dtype=torch.float64).mul(2).sub(1).cuda()
+    for cfg in ({"type": "ILU"}, {"type": "ILU", "diagonalBased": True}):
+        s, want = gb.Solver(A, cfg), gb.Solver(A, {**cfg, "kernel": "levels"})
+        assert s.sweepKernel(coef) == name + " factor"
+        for dt in (torch.float32, torch.float64)[0 if coef == F32 else 1:]:
+            for off in (0, 1):  # the second: not 16-byte aligned
+                b = b64.to(dt)[off:off + n]
+                x, y = (torch.zeros(n + 1, dtype=dt, device="cuda")[off:off + n] for _ in range(2))
+                s.solve(x, b)
+                want.solve(y, b)
+                assert torch.equal(x, y)
