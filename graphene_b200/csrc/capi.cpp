@@ -16,10 +16,12 @@ struct gr_host_matrix {
 };
 
 struct gr_matrix {
-  std::unique_ptr<gr::DeviceMatrix> d;
+  std::shared_ptr<gr::DeviceMatrix> d;
 };
 
+// Holds its matrix: the two may be destroyed in either order.
 struct gr_solver {
+  std::shared_ptr<gr::DeviceMatrix> d;
   std::unique_ptr<gr::SolverTree> s;
 };
 
@@ -503,7 +505,7 @@ int gr_matrix_create(gr_host_matrix* h, gr_matrix** out) {
   return guarded([&] {
     need(h, "host matrix");
     need(out, "out");
-    auto d = std::make_unique<gr::DeviceMatrix>(h->m);
+    auto d = std::make_shared<gr::DeviceMatrix>(h->m);
     *out = new gr_matrix{std::move(d)};
   });
 }
@@ -638,7 +640,7 @@ int gr_solver_create(gr_matrix* A, const char* json, gr_solver** out) {
     need(json, "json");
     need(out, "out");
     auto s = gr::SolverTree::create(*A->d, json);
-    *out = new gr_solver{std::move(s)};
+    *out = new gr_solver{A->d, std::move(s)};
   });
 }
 

@@ -439,7 +439,8 @@ int gr_compose_vector(gr_matrix* A, const void* tile_ordered, void* natural, gr_
  * IterativeRefinement | restarter, nested "preconditioner" /
  * "innerSolver"); comments are allowed. Construction performs the ILU
  * factorisation as the reference's ilu::Solver constructor does
- * (ilu/Solver.cpp:44-51). */
+ * (ilu/Solver.cpp:44-51). A solver keeps its matrix alive: the two handles
+ * may be destroyed in either order. */
 int gr_solver_create(gr_matrix* A, const char* json, gr_solver** out);
 void gr_solver_destroy(gr_solver* s);
 
