@@ -528,6 +528,9 @@ struct DeviceMatrix {
                        RingKind kind = RingKind::Ilu, bool records = false);
 
   std::map<std::tuple<int, bool, i32>, std::unique_ptr<DirectPlan>> directPlans;  // [(kind, dilu, warps)]
+  // directShape for this matrix on its device, worked out once.
+  const DirectShape& directShapeFor(RingKind kind, DType vec);
+  std::map<std::pair<int, int>, DirectShape> directShapes;  // [(kind, vectors)]
   // nullptr when the direct kernels cannot run this sweep, or a block that
   // copies `depth` steps ahead over double vectors does not fit smemMax; the
   // tables are then not kept on the device.

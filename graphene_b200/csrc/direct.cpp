@@ -3,6 +3,7 @@
 // device.hpp for the layout.
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 
 #include "device.hpp"
 
@@ -464,27 +465,28 @@ double rowsPerLevel(const HostMatrix& H) {
 // 65.6 -> 43.2, two 47.4; below, 96/300: 39.6 -> 28.0, four 31.9). Then two
 // while a level fills them (128/512, 89 rows: 46.3 -> 39.1; 160/600, 119 rows:
 // 118.9 -> 100.1, one 108.7), else one (64/512: 18.6 -> 10.4; 128/1024: 41.2 ->
-// 35.0, two 41.0). Depth: 8, or 4 where only then all tiles are resident
-// (160/1370: 91.7 -> 80.0, with 8 103.7). A last wave that is not full costs
-// more than it does the ring, whose blocks hold less: ring from 1.3 waves on
-// (192/1184, 1.6: 125.9, direct 148; 176/2000, 1.5: 98.8, 108.3; 176/4096,
-// 2.3: 90, 105), for levels of 25 to 40 rows from two on (140x151x174/4944,
-// 2.4: 74.0, 78.9; 176x176x130/6185, 3.0: 84.1, 90.7; 144/3000, 1.6: 73.8 ->
-// 63.9); with two full waves they break even (192/2368: 104.9, 104.8).
-// Narrower levels cost the ring its hand-overs and always run direct (2048^2
-// in 2368 tiles, 20 rows: 150.2 -> 91.5, a chain of 2^20 rows in 1024: 1154 ->
-// 207). Levels of a step of two warps and a little more, five or six tiles an
-// SM, data beyond L2: ring (144/800: 59.5, 69.7; 128/700: 49.0, 51.4; the same
-// in L2, m100/700: 30.8 -> 22.7).
+// 35.0, two 41.0); tiles of several waves with levels beyond 80 rows, two
+// (192/1184: 125.9 -> 125.5, one 148). Depth: 8, or 4 where that saves a wave
+// (160/1370: 91.7 -> 80.0, with 8 103.7; 176/4096, 1.5 waves for 2.3: 99.3,
+// with 8 104.9; in as many waves, 192/2368: 109.4, with 8 104.8, ring 104.9).
+// Direct in several waves ran at 0.84 to 1.10 of the ring's time over 60
+// grids, with no line between them, and its set-up takes half as long, so it
+// is kept (176x160x172/2595: 104.2 -> 88; 176/2000: 98.8 -> 108). Ring for
+// wide levels on five to seven tiles an SM with data beyond L2, if its blocks
+// then all fit beside a ring of 16 KB (144/800: 59.5, 69.7; 140/850: 57.2, 64;
+// 150/1000: 67.7, 78; not where it needs a second wave, 150/900: 95.0 -> 81,
+// nor in L2, m100/700: 30.8 -> 22.7).
+// Narrow levels cost the ring its hand-overs (2048^2 in 2368 tiles, 20 rows:
+// 150.2 -> 91.5, a chain of 2^20 rows in 1024: 1154 -> 207).
 //
 // ILU, double vectors. A step costs twice the cycles, so that few resident
 // warps no longer hide DRAM. Float coefficients: ring beyond about 165 MB
-// (160/600: 151.6, direct 160.7; 160/1370: 138.3, 154; 144/1300: 89.9, 110;
-// below 128/1024: 66.4 -> 46.9), for levels of 25 to 40 rows from 2.1 waves on
-// (160/4096: 91, 100; 144/3000: 114 -> 87); beyond half of L2 for wide levels
-// on up to 2.5 tiles an SM (128/148: 107.5, 125; 112/300: 73.5, 89; 96/148:
-// 51.4 -> 43) and on little more than four (130x107x112/609: 51.2, 59.5;
-// 112/750: 45.1, 45.3). Double coefficients: ring for more than one and a
+// with up to ten tiles an SM and more than 40 rows a level (160/600: 151.6,
+// direct 160.7; 160/1370: 138.3, 154; 144/1300: 89.9, 110; more tiles,
+// 160/2048: 110 -> 102; below, 128/1024: 66.4 -> 46.9); beyond half of L2 for
+// wide levels on up to 2.5 tiles an SM (128/148: 107.5, 125; 112/300: 73.5,
+// 89; 96/148: 51.4 -> 43) and on little more than four (130x107x112/609: 51.2,
+// 59.5; 112/750: 45.1, 45.3). Double coefficients: ring for more than one and a
 // quarter waves, for up to four tiles an SM (wide levels: five) beyond L2
 // (128/148: 105.5, 125; 112/300: 73.9, 95; 112/450: 47.3, 52.1; 120/640: 53.4,
 // 59.9; 128/512: 57.4, 56.3; below, 96/148: 49.3 -> 43.3) and from three on
@@ -509,7 +511,7 @@ DirectShape directShape(const HostMatrix& H, RingKind kind, DType coefficients, 
   const double t = static_cast<double>(H.P) / numSMs, rows = rowsPerLevel(H);
   // Waves of blocks with room for second triples, copying d steps ahead.
   const i64 vs = static_cast<i64>(dtypeSize(vec)), rec = f32 ? 44 : 72;
-  auto waves = [&](i32 warps, i32 d) {
+  auto waves = [&](i32 warps, i32 d, i64 vs) {
     i64 steps = 0;  // of the longest tile, at most
     for (i32 T = 0; T < H.P; ++T) {
       const i64 nRows = H.tileStart[T + 1] - H.tileStart[T];
@@ -524,30 +526,43 @@ DirectShape directShape(const HostMatrix& H, RingKind kind, DType coefficients, 
     i32 warps = t <= 2 ? 4 : rows > 45 ? 2 : 1;
     if (!f32) {
       warps = t <= 2 && rows > 150 ? 4 : t > 4 ? 1 : 0;
-      if (warps == 0 || waves(warps, kDirectGsDepth) > 1) return {};
+      if (warps == 0 || waves(warps, kDirectGsDepth, vs) > 1) return {};
     }
     return {warps, kDirectGsDepth};
   }
-  const i32 warps = t <= 1   ? (rows > 40 ? 4 : 2)
-                    : t <= 2 ? (rows > 80 ? 4 : 2)
-                    : t <= 4 ? (rows > 40 ? 2 : 1)
-                             : (t <= 6 && rows > 64 ? 2 : 1);
-  const i32 depth = waves(warps, 8) > 1 && waves(warps, 4) <= 1 ? 4 : 8;
-  const double w = waves(warps, depth);
+  const i32 warps = t <= 1                               ? (rows > 40 ? 4 : 2)
+                    : t <= 2                             ? (rows > 80 ? 4 : 2)
+                    : t <= 4                             ? (rows > 40 ? 2 : 1)
+                    : t <= 6                             ? (rows > 64 ? 2 : 1)
+                    : rows > 80 && waves(1, 8, 4) > 1.3 ? 2
+                                                         : 1;
+  const double w8 = waves(warps, 8, vs), w4 = waves(warps, 4, vs);
+  const i32 depth = w8 > 1 && std::ceil(w4) < std::ceil(w8) ? 4 : 8;
   // A seven-point grid's coefficients and two vectors.
   const double mb = static_cast<double>(H.n) * (f32 ? 50 + 2 * vs : 116) * 1e-6;
   bool ring;
   if (!f32) {
-    ring = w > 1.25 || (rows > 40 && t <= (rows > 64 ? 5 : 4) && (mb > 120 || t > 3));
+    ring = (depth == 4 ? w4 : w8) > 1.25 || (rows > 40 && t <= (rows > 64 ? 5 : 4) && (mb > 120 || t > 3));
   } else if (vec == DType::F64) {
-    ring = (mb > 165 && (rows > 40 || (rows > 25 && w > 2.1))) ||
+    ring = (mb > 165 && rows > 40 && t <= 10) ||
            (mb > 66 && ((rows > 80 && t <= 2.5) || (rows > 55 && t > 4 && t <= 5)));
   } else {
-    ring = ((w < 1.96 || w > 2.02) && ((rows > 40 && w > 1.3) || (rows > 25 && w > 2))) ||
-           (mb > 100 && rows > 64 && rows < 90 && t > 4.5 && t <= 6);
+    // 17.5 KB: a ring of 16, its barriers and level table.
+    const double room = static_cast<double>(smemPerSM) / std::ceil(t) - 4.0 * static_cast<double>(H.maxTileRows) - 1024;
+    ring = mb > 100 && rows > 64 && t > 4.5 && room > 17.5e3;
   }
   if (ring) return {};
   return {warps, depth};
+}
+
+const DirectShape& DeviceMatrix::directShapeFor(RingKind kind, DType vec) {
+  const auto [at, made] = directShapes.try_emplace({static_cast<int>(kind), static_cast<int>(vec)});
+  if (made) {
+    int perSM = 0;
+    GR_CUDA(cudaDeviceGetAttribute(&perSM, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device));
+    at->second = directShape(*host, kind, vt, vec, numSMs, perSM);
+  }
+  return at->second;
 }
 
 DirectPlan* DeviceMatrix::directPlan(RingKind kind, bool dilu, i32 warps, i32 depth, size_t smemMax) {

@@ -70,12 +70,6 @@ void printStats(const SolverConfig& c, const DeviceMatrix& A, const gr_stats& st
                st.iterations, st.converged ? "true" : "false", st.singular ? "true" : "false");
 }
 
-DirectShape directShapeFor(const DeviceMatrix& A, RingKind kind, DType vec) {
-  int perSM = 233472;
-  GR_CUDA(cudaDeviceGetAttribute(&perSM, cudaDevAttrMaxSharedMemoryPerMultiprocessor, A.device));
-  return directShape(*A.host, kind, A.vt, vec, A.numSMs, perSM);
-}
-
 // nullptr also when the tables exceed their limits or memory: the other
 // kernels need less.
 DirectPlan* directPlanOrNull(DeviceMatrix& A, RingKind kind, bool dilu, i32 warps, i32 depth, size_t smemMax) {
@@ -114,8 +108,8 @@ class IluNode : public Node {
       kernel_ = 5;
     }
     if (direct && c.iluKernel == 0 && !ringOptions(c)) {
-      const DirectShape own = directShapeFor(A, RingKind::Ilu, A.vt);
-      const DirectShape wide = directShapeFor(A, RingKind::Ilu, DType::F64);
+      const DirectShape own = A.directShapeFor(RingKind::Ilu, A.vt);
+      const DirectShape wide = A.directShapeFor(RingKind::Ilu, DType::F64);
       depth_ = own.depth;
       wideDepth_ = wide.warps > 0 ? wide.depth : own.depth;
       if (own.warps > 0)
@@ -269,7 +263,8 @@ class IluNode : public Node {
   // two consecutive tiles a block with four compute warps when the tiles
   // fill at least two waves of one-tile blocks and the grouped blocks take
   // no more waves. The waiting and producer warps' per-level work is then
-  // shared by two tiles; on B200 at 192^3 with 2368 tiles that ran the
+  // shared by two tiles; on B200 at 192^3 with 2368 tiles and "kernel": "ring"
+  // (the automatic choice there is the direct kernel) that ran the
   // substitution in 104.4 us against 111.8 (MPIR 121.7 against 125.0 ms),
   // while at 2048 tiles, where grouping adds a wave, it ran slower. FP64
   // coefficients keep one tile a block (their slices halve the blocks per
@@ -329,7 +324,7 @@ class GsNode : public Node {
     // vector type): one ring with every entry, and one with the lower
     // entries only for sweeps that start from x = 0.
     if (c.gsKernel == 0 && c.ringRecords && c.warpsPerBlock == 1 && !c.gsPairRows) {
-      const i32 warps = directShapeFor(A, RingKind::GaussSeidel, A.vt).warps;
+      const i32 warps = A.directShapeFor(RingKind::GaussSeidel, A.vt).warps;
       const size_t smemMax = static_cast<size_t>(maxDynamicSmem(A));
       auto plan = [&](RingKind kind) { return directPlanOrNull(A, kind, false, warps, kDirectGsDepth, smemMax); };
       if (warps > 0) direct_ = plan(RingKind::GaussSeidel);
@@ -501,7 +496,7 @@ class GsNode : public Node {
     if (Wc == W) return W;
     if (!(W == DType::F32 && Wc == DType::F64))
       fail(GR_EUNSUPPORTED, "GaussSeidel workingType must be the vectors' type or float64 over float32 vectors");
-    if (!levelBlocks()) fail(GR_EUNSUPPORTED, "a GaussSeidel workingType other than the vectors' needs the ring kernel");
+    if (!levelBlocks()) fail(GR_EUNSUPPORTED, "a GaussSeidel workingType other than the vectors' needs the direct or ring kernel");
     return Wc;
   }
   // Level-ring sweeps: the first takes its right-hand side from `first`
@@ -1159,6 +1154,7 @@ class Tree : public SolverTree {
     if (reps < 1 || reps > 100000) fail(GR_EINVAL, "reps must be 1..100000");
     if (cfg_->type != "ILU" && !(cfg_->type == "GaussSeidel" && cfg_->numFixedIterations > 0))
       fail(GR_EUNSUPPORTED, "repeated timing is for ILU and fixed-sweep Gauss-Seidel solvers");
+    root_->prepare(xt);
     GR_CUDA(cudaEventRecord(e0_, A_.stream));
     for (int i = 0; i < reps; ++i) root_->solve(x, b, xt, nullptr);
     GR_CUDA(cudaEventRecord(e1_, A_.stream));

@@ -41,6 +41,7 @@ def mesh(n, tiles):
     (lambda: grid(96, 560), ILU, F64, F64),
     (lambda: grid(112, 300), ILU, F64, F64),
     (lambda: grid(112, 300), ILU, F32, F64),
+    (lambda: grid(128, 700), ILU, F32, F32),
 ])
 def test_ring_where_it_is_faster(make, sweep, coef, vec):
     assert shape(make(), sweep, coef, vec) == (0, 0)
@@ -66,12 +67,11 @@ def test_direct_where_it_is_faster(make, sweep, coef, vec, want):
     assert shape(make(), sweep, coef, vec) == want
 
 
-def test_last_wave():
-    """Float tiles in one and a half waves take the ring, in less or nearly two
-    the direct kernel, with four steps ahead where that makes one wave of more."""
+def test_depth_by_waves():
+    """Four steps ahead where the tiles then need a wave less."""
     h = grid(96, 592)  # 11 tiles an SM with 8 steps ahead, 15 with 4
-    got = {sms: shape(h, ILU, F32, F32, sms) for sms in (54, 45, 36, 27)}
-    assert got == {54: (1, 8), 45: (1, 4), 36: (0, 0), 27: (1, 8)}
+    got = {sms: shape(h, ILU, F32, F32, sms) for sms in (54, 45, 36, 27, 20)}
+    assert got == {54: (1, 8), 45: (1, 4), 36: (1, 8), 27: (1, 8), 20: (1, 4)}
 
 
 @pytest.mark.gpu
