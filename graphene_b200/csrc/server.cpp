@@ -40,8 +40,9 @@ i64 estimateFootprint(const HostMatrix& H, const std::string& json, DType t) {
                         12 * upperLevels + 2 * words;
   const i64 gsDirect = 2 * (record * H.lowerRows8 + 12 * lowerLevels + words) + 4 * H.numHaloTotal;
   const i64 direct = std::max(iluDirect, gsDirect);
-  // Double vectors over float coefficients may keep a ring beside them.
-  const i64 sweeps = vs == 4 && t == DType::F64 ? stream + direct : std::max(stream, direct);
+  // Double vectors over float coefficients (also by workingType) may keep a
+  // ring beside them.
+  const i64 sweeps = vs == 4 ? stream + direct : std::max(stream, direct);
   const i64 factors = m * vs + n * vs;
   const i64 vectors = 16 * n * std::max<i64>(8, static_cast<i64>(dtypeSize(t)));     // Krylov, MPIR, staging
   return sell + rows + localCrs + sweeps + factors + vectors + (i64(4) << 20);
