@@ -350,7 +350,7 @@ def other_configs(gb, peak):
             out["convdiff128_gs_sweep"] = {"ms": ms, "bytes_per_sweep": byts,
                                            "GBs": byts / (ms * 1e-3) / 1e9,
                                            "frac_of_hbm": byts / (ms * 1e-3) / 1e9 / peak,
-                                           "kernel": "gsWarpRingKernel (one warp per tile)"}
+                                           "kernel": gs1.sweepKernel(gb.FLOAT32)}
             del gs1, xg
         del A
     # 100^3 LDU mesh (jittered, permuted), Gauss-Seidel PBiCGStab to 1e-8,
@@ -533,7 +533,7 @@ def serving(gb, requests=10000, slots=16, seed=7, rate_requests=2000, cold_reque
 
 def batching(gb, systems=64, seed=11, reps=3):
     """Many uneven systems: 7-point variable-coefficient Poisson (sigma 1),
-    grid edge U{16..48}, FP32 PBiCGStab + ILU(0) (ring kernel) to 1e-6,
+    grid edge U{16..48}, FP32 PBiCGStab + ILU(0) (automatic kernel) to 1e-6,
     host vectors in and out. One batch (gr_batch_solve_host: every launch
     covers all systems) against the same systems solved one after another
     by resident solvers (gr_solve_host); best of `reps` wall-clock passes,
@@ -542,7 +542,7 @@ def batching(gb, systems=64, seed=11, reps=3):
     import numpy as np
     rng = np.random.default_rng(seed)
     cfg = {"type": "PBiCGStab", "maxIterations": 1000, "relResidual": 1e-6,
-           "preconditioner": {"type": "ILU", "kernel": "ring"}}
+           "preconditioner": {"type": "ILU"}}
     hs, bs = [], []
     for k in range(systems):
         L = int(rng.integers(16, 49))
@@ -878,15 +878,18 @@ def main():
     # Dominant kernel: two ILU(0) applications and two SpMVs per inner iteration.
     inner = st.innerIterations
     if 2 * inner * ilu_ms >= 2 * inner * spmv_ms:
-        dom = ("ilu0_apply", "iluDirectKernel", ilu_bytes, ilu_ms)
+        names = {"direct": "iluDirectKernel", "ring": "iluRingKernel"}
+        chosen = ilu.sweepKernel(gb.FLOAT32).split()[0]
+        dom = ("ilu0_apply", names.get(chosen, chosen), ilu_bytes, ilu_ms)
     else:
         dom = ("spmv", "spmvDotKernel", spmv_bytes, spmv_ms)
     # DRAM bytes per launch of the dominant kernel from the committed ncu
-    # summary (a 160^3 capture of the kernel the 192^3 solve runs, scaled by
-    # rows to one 192^3 launch).
+    # summary of iluDirectKernel (a 160^3 capture in the four-steps-ahead shape;
+    # its reads scaled by rows to one 192^3 launch, which copies eight steps
+    # ahead, plus the whole result, of which the capture left most in L2).
     traffic = None
     tf = ROOT / "profiles" / "ilu_direct_var_poisson_160.md"
-    if dom[0] == "ilu0_apply" and a.grid == 192 and tf.exists():
+    if dom[1] == "iluDirectKernel" and a.grid == 192 and tf.exists():
         import re
         hit = re.search(r"traffic_bytes_192: (\d+)", tf.read_text())
         traffic = int(hit.group(1)) if hit else None

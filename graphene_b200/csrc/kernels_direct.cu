@@ -318,19 +318,14 @@ __device__ __forceinline__ void tileStore(X* __restrict__ y, int base, int nRows
   }
 }
 
-template <int WARPS>
-__device__ __forceinline__ void levelBarrier() {
-  if (WARPS == 1) __syncwarp();
-  else __syncthreads();
-}
-
 // 16-byte units of a tile's stream that its block keeps on their way to L2
 // beyond its copies. With the stream in DRAM the copies alone, DEPTH steps
 // ahead, leave too few bytes in flight: on B200, L2 flushed, 8 KB ahead ran
 // the 128^3 / 1024 ILU(0) in 41.3 us against 45.9 without (float64 63.6
 // against 68.3), 96^3 / 432 in 30.8 against 31.6, the 100^3 mesh's two sweeps
-// in 51.6 against 56.1; with it in L2 nothing changes (35.1 / 34.9 us; float64
-// 49.3 / 53.4). 4 and 16 KB ran within 3 us of it, a whole tile ahead slower.
+// in 51.6 against 56.1. Back to back, the 128^3 stream stays in L2 and nothing
+// changes (35.1, 34.9 without); the float64 one does not (49.3, 53.4 without).
+// 4 and 16 KB ran within 3 us of it, a whole tile ahead slower.
 // Streams of less than 32 MB (kDirectFetchUnits) stay in L2 between a solve's
 // applications, and the 32^3 / 64 one takes 8.2 us without and up to 10 with
 // the prefetch, so they go without.

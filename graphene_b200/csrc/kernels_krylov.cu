@@ -158,7 +158,9 @@ __global__ void __launch_bounds__(256) bicgUpdateKernel(W* __restrict__ x, const
   __shared__ double smem[64];
   const SegPos sp = segPos(seg, n);
   st += sp.sys;
-  const int done = st->done;  // tested after the first loads, not before them
+  // Tested after the first loads, not before them: a finished system of a
+  // batch pays for one round of loads so that the others do not wait twice.
+  const int done = st->done;
   const W al = cvt<W>(st->alpha), om = cvt<W>(st->omega);
   const int nk = st->normKind;
   double v[2] = {redIdentity(normOp(nk)), 0.0};
