@@ -489,8 +489,9 @@ double rowsPerLevel(const HostMatrix& H) {
 // 59.5; 112/750: 45.1, 45.3). Double coefficients: ring for more than one and a
 // quarter waves, for up to four tiles an SM (wide levels: five) beyond L2
 // (128/148: 105.5, 125; 112/300: 73.9, 95; 112/450: 47.3, 52.1; 120/640: 53.4,
-// 59.9; 128/512: 57.4, 56.3; below, 96/148: 49.3 -> 43.3) and from three on
-// already in L2 (96/560: 32.9, 35.0; m100/700: 32.8, 37.0); else direct
+// 59.9; 128/512: 57.4, 56.3; below, 96/148: 49.3 -> 43.3) or up to five whose
+// rings all fit (101x122x116/599: 49.2, 57.5; not 130x107x112/609: 71.4 ->
+// 61.6) and from three on already in L2 (96/560: 32.9, 35.0; m100/700: 32.8, 37.0); else direct
 // (128/1024: 67.0 -> 49.2, 96/1200: 47.3 -> 33.5).
 //
 // Gauss-Seidel (two sweeps; a row costs a division and up to six entries).
@@ -540,15 +541,19 @@ DirectShape directShape(const HostMatrix& H, RingKind kind, DType coefficients, 
   const i32 depth = w8 > 1 && std::ceil(w4) < std::ceil(w8) ? 4 : 8;
   // A seven-point grid's coefficients and two vectors.
   const double mb = static_cast<double>(H.n) * (f32 ? 50 + 2 * vs : 116) * 1e-6;
+  // What a level ring's block may use beside its x when all tiles are resident
+  // at once. Rings take 16 KB (float) or twice their widest level (double),
+  // and 1.5 KB of barriers and level table.
+  const double room = static_cast<double>(smemPerSM) / std::ceil(t) -
+                      static_cast<double>(vs) * static_cast<double>(H.maxTileRows) - 1024;
   bool ring;
   if (!f32) {
-    ring = (depth == 4 ? w4 : w8) > 1.25 || (rows > 40 && t <= (rows > 64 ? 5 : 4) && (mb > 120 || t > 3));
+    ring = (depth == 4 ? w4 : w8) > 1.25 || (rows > 40 && t <= (rows > 64 ? 5 : 4) && (mb > 120 || t > 3)) ||
+           (rows > 40 && t <= 5 && mb > 120 && room > 23.3e3);
   } else if (vec == DType::F64) {
     ring = (mb > 165 && rows > 40 && t <= 10) ||
            (mb > 66 && ((rows > 80 && t <= 2.5) || (rows > 55 && t > 4 && t <= 5)));
   } else {
-    // 17.5 KB: a ring of 16, its barriers and level table.
-    const double room = static_cast<double>(smemPerSM) / std::ceil(t) - 4.0 * static_cast<double>(H.maxTileRows) - 1024;
     ring = mb > 100 && rows > 64 && t > 4.5 && room > 17.5e3;
   }
   if (ring) return {};

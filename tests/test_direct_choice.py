@@ -40,6 +40,7 @@ def mesh(n, tiles):
     (lambda: gb.generate3DPoissonMatrix(F32, 109, 80, 107, 931, gb.PART_RCB), GS, F64, F64),
     (lambda: grid(96, 560), ILU, F64, F64),
     (lambda: grid(112, 300), ILU, F64, F64),
+    (lambda: gb.generate3DPoissonMatrix(F32, 101, 122, 116, 599, gb.PART_RCB), ILU, F64, F64),
     (lambda: grid(112, 300), ILU, F32, F64),
     (lambda: grid(128, 700), ILU, F32, F32),
 ])
@@ -56,6 +57,7 @@ def test_ring_where_it_is_faster(make, sweep, coef, vec):
     (lambda: mesh(80, 256), ILU, F64, F64, (4, 8)),
     (lambda: grid(96, 148), ILU, F64, F64, (4, 8)),
     (lambda: grid(96, 1200), ILU, F64, F64, (1, 4)),
+    (lambda: gb.generate3DPoissonMatrix(F32, 130, 107, 112, 609, gb.PART_RCB), ILU, F64, F64, (1, 8)),
     (lambda: grid(64, 64), GS, F32, F32, (4, 4)),
     (lambda: grid(96, 432), GS, F32, F64, (2, 4)),
     (lambda: grid(64, 512), GS, F32, F32, (1, 4)),
