@@ -443,7 +443,7 @@ struct DirectPlan {
   bool longForward = false;  // ILU: the forward sweep has rows of more than three entries
   i32 warps = 1, maxSteps = 0;
   i64 records = 0, units = 0, maxRows = 0, maxXSlots = 0;
-  bool factors = false;
+  bool factors = false;  // with the tables of the fused factorisation (ILU)
   DBuf levelStart, levels, transposed, transposed2;
   DBuf src, src2, tail, tail2, steps, stepStart, stepRecord, stepUnit, haloStart, haloSrc;
 };

@@ -596,8 +596,13 @@ DirectPlan* DeviceMatrix::directPlan(RingKind kind, bool dilu, i32 warps, i32 de
         R->src2.upload(D.src2);
         R->tail2.upload(D.tail2);
       }
-      R->factors = D.factors;
-      if (D.factors) {
+      // Chains, whose levels are single rows, on more than a tile an SM
+      // factorise apart: the many streams of the fused factorisation cost more
+      // than its launches save (2^20 rows in 1024 tiles: 2.8 ms, with separate
+      // kernels 1.5; in 256 tiles 5.5 and 4.9; 65,536 rows in 64 tiles, one an
+      // SM: 0.9 and 1.2).
+      R->factors = D.factors && (P <= numSMs || rowsPerLevel(*host) >= 2);
+      if (R->factors) {
         R->levelStart.upload(D.levelStart);
         R->levels.upload(D.levels);
         R->transposed.upload(D.transposed);

@@ -145,12 +145,7 @@ class IluNode : public Node {
       else if (c.iluKernel == 1 && tmaFits) kernel_ = 1;
       else fail(GR_EUNSUPPORTED, "the requested ILU kernel does not fit this matrix's tiles in shared memory");
     }
-    // Chains, whose levels are single rows, on more than a tile an SM: the
-    // many streams of the fused factorisation cost more than its launches
-    // save (2^20 rows in 1024 tiles: 2.8 ms, with separate kernels 1.5; in 256
-    // tiles 5.5 and 4.9; 65,536 rows in 64 tiles, one an SM: 0.9 and 1.2).
-    fusedFactor_ = kernel_ == 6 && direct_->factors && directFactorSmem(*direct_, A.vt) <= smemMax &&
-                   (A.P <= A.numSMs || rowsPerLevel(*A.host) >= 2);
+    fusedFactor_ = kernel_ == 6 && direct_->factors && directFactorSmem(*direct_, A.vt) <= smemMax;
     if (!fusedFactor_) inv_.alloc(A.n * vs);
     if (kernel_ == 6) {
       stream_.alloc(directBytes(*direct_));
